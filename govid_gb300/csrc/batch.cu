@@ -37,7 +37,7 @@ struct Slot {
   // per macroblock: whether its inter prediction waits for the previous
   // frame's intra stage; then two intra progress bytes (large tiles)
   uint8_t* dep = nullptr;
-  uint8_t* symLog = nullptr;   // the entropy stage's symbol log, kSymPerMB bytes per macroblock
+  uint8_t* symLog = nullptr;   // the entropy stage's symbol log (symLogBytes)
   uint32_t* symOff = nullptr;  // per macroblock: its first symbol in its tile's log
   bool alloc(size_t mbs) {
     return cudaMalloc(&dep, 3 * mbs) == cudaSuccess && cudaMalloc(&rec, mbs * sizeof(MBRec)) == cudaSuccess &&
@@ -46,7 +46,7 @@ struct Slot {
            cudaMalloc(&lv, mbs * sizeof(int16_t)) == cudaSuccess &&
            cudaMalloc(&intra, 2 * mbs * sizeof(uint32_t)) == cudaSuccess &&
            cudaMalloc(&ts, mbs * sizeof(TileStat)) == cudaSuccess &&
-           cudaMalloc(&symLog, mbs * kSymPerMB) == cudaSuccess &&
+           cudaMalloc(&symLog, symLogBytes(mbs)) == cudaSuccess &&
            cudaMalloc(&symOff, mbs * sizeof(uint32_t)) == cudaSuccess;
   }
   void release() {
@@ -61,7 +61,7 @@ struct Slot {
     cudaFree(symOff);
   }
   static size_t bytes(size_t mbs) {
-    return mbs * (sizeof(MBRec) + kCoefPerMB * 4 + 4 + 2 + 8 + sizeof(TileStat) + 3 + kSymPerMB + 4);
+    return mbs * (sizeof(MBRec) + kCoefPerMB * 4 + 4 + 2 + 8 + sizeof(TileStat) + 3 + 4) + symLogBytes(mbs);
   }
 };
 
@@ -950,7 +950,6 @@ int Engine::planRound(const std::vector<int>& ids, const std::vector<int>* maxFr
     fd.tileStat = sl.ts;
     fd.symLog = sl.symLog;
     fd.symOff = sl.symOff;
-    fd.symPerMB = kSymPerMB;
     fd.status = reinterpret_cast<int32_t*>(d + R.oStat) + di;
     fd.gate = gateDesc >= 0 ? reinterpret_cast<const int32_t*>(d + R.oStat) + gateDesc : nullptr;
     fd.dep = sl.dep;

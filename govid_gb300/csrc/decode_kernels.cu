@@ -1,15 +1,12 @@
 // GB300 (sm_103a) EBIV decode kernels.
 //
 // Stage A  kEntropy   one warp per tile, up to four tiles of one frame per
-//                     CTA sharing the frame's symbol tables: the tile's
-//                     4-state interleaved rANS chain (ebiv/rans.go:270-304)
-//                     drives the macroblock grammar
-//                     (ebiv/decode_intra.go:121-167, ebiv/decode_inter.go:8-62,
-//                     ebiv/residual.go:79-126, ebiv/mv.go) and emits one
-//                     MBRec per macroblock plus sparse levels.  The warp runs
-//                     the chain in lockstep; a symbol costs one shared-memory
-//                     lookup (slot bucket -> symbol, start, frequency) except
-//                     in the few buckets a symbol boundary crosses.
+//                     CTA sharing the frame's symbol tables: one thread runs
+//                     the tile's symbol chain (symbol_chain.h) into a log,
+//                     from which kParseMB makes one MBRec per macroblock plus
+//                     sparse levels; a tile that the chain leaves (a symbol
+//                     fails, the log is full) is decoded by the whole warp in
+//                     lockstep, records and levels included (fullChain).
 // Stage B1 kInterRecon one warp per macroblock of an inter frame: motion
 //                     compensation (ebiv/motioncomp.go) from the last or
 //                     golden reference plus dequantized inverse DCT residual
@@ -24,9 +21,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 
 #include "gpu_types.h"
+#include "symbol_chain.h"
 
 namespace ebiv {
 namespace dev {
@@ -38,6 +37,8 @@ constexpr unsigned kFull = 0xffffffffu;
 // bandOf(i) * kNumPrevClass * 64 (bits 8-19).  One entry past each scan is
 // zero, so the next position's entry can always be loaded.
 __constant__ uint32_t cScanRow[3][257];
+// The same positions for lanes that read different ones.
+__device__ uint8_t gScan[3][256];
 // 2^13-scaled DCT-II basis, [k*n + i], per transform size.  Global memory:
 // the transforms read it with a different index in every lane, which the
 // L1 path serves in one pass and the constant cache would serialise.
@@ -59,106 +60,77 @@ __device__ __forceinline__ int16_t clampMV(int v) {
 // ---------------------------------------------------------------------------
 // Stage A: entropy decode
 // ---------------------------------------------------------------------------
-// Symbol tables, built once per CTA for the frame whose tiles the CTA
-// decodes.  bucket[c*64+b] describes the symbol s of context c whose range
-// holds slot b*64: start (bits 0-11), frequency (12-24), s (25-28), a flag
-// (29) when a later symbol starts inside the bucket (the decoder then walks
-// sym[]), and a flag (30) for an unused context, whose entry decodes as the
-// identity so the chain stays well defined after the error.  sym[c*16+s]
-// packs start | frequency << 16 for the walk.
-constexpr uint32_t kBImpure = 1u << 29, kBUnused = 1u << 30;
-struct EntropyTables {
-  uint32_t bucket[kNumContexts * 64];
-  uint32_t sym[kNumContexts * 16];
-};
 constexpr int kRowMax = 128;  // tiles at most this many macroblocks wide pass vector rows in shared memory
 struct WarpRows {
   uint32_t mv[2][kRowMax];  // packed vectors of a pass's last row, by pass parity
 };
 
+// One warp per context in turn: lane s holds where symbol s starts and
+// writes its entry, then each lane finds two buckets' symbols among them.
 __device__ __forceinline__ void buildTables(EntropyTables& T, const DeviceTables& src, int tid, int nthreads) {
-  for (int i = tid; i < kNumContexts * 16; i += nthreads) {
-    const int c = i >> 4, sidx = i & 15;
-    const uint32_t st = src.start[c][sidx], nx = src.start[c][sidx + 1];
-    T.sym[i] = (st == 0xFFFFu || nx == 0xFFFFu) ? 0xFFFFu : (st | ((nx - st) << 16));
-  }
-  for (int i = tid; i < kNumContexts * 64; i += nthreads) T.bucket[i] = (kM << 12) | kBUnused;
-  __syncthreads();
-  // Each (context, symbol) pair fills the buckets whose first slot it covers.
-  for (int i = tid; i < kNumContexts * 16; i += nthreads) {
-    const int c = i >> 4, sidx = i & 15;
-    if (!src.used[c]) continue;
-    const uint32_t st = src.start[c][sidx], nx = src.start[c][sidx + 1];
-    if (st == 0xFFFFu || nx == 0xFFFFu || nx <= st) continue;
-    for (uint32_t b = (st + 63) >> 6; b < 64 && (b << 6) < nx; b++)
-      T.bucket[c * 64 + b] = st | ((nx - st) << 12) | ((uint32_t)sidx << 25) | (nx < ((b + 1) << 6) ? kBImpure : 0u);
+  const int lane = tid & 31;
+  if (tid < kBlockKinds) T.block[tid] = blockEntry(tid);
+  for (int c = tid >> 5; c < kNumContexts; c += nthreads >> 5) {
+    const int places = c == ctxSign ? 4 : 1;
+    uint4* const e = T.entry + rowOf(c) / 16 + 4 * lane;
+    if (!src.used[c]) {
+      for (int k = 0; k < places; k++) e[k] = e[4 * 32 + k] = unusedEntry();
+      continue;
+    }
+    const uint32_t start = lane < 17 ? (uint32_t)src.start[c][lane] : 0xFFFFu;
+    const uint32_t after = __shfl_down_sync(kFull, start, 1);
+    if (lane < kSymbols)
+      T.symbol[c * kSymbols + lane] = start < kM ? symbolEntry(c, lane, start, after - start, 0u) : sentinelEntry();
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const uint32_t b = (uint32_t)(lane + 32 * h);
+      uint32_t s = 0, st = 0, nx = kM;
+#pragma unroll
+      for (int k = 1; k < 16; k++) {
+        const uint32_t v = __shfl_sync(kFull, start, k);
+        if (v <= b << 6) {
+          s = (uint32_t)k;
+          st = v;
+        } else {
+          nx = min(nx, v);
+        }
+      }
+      for (int k = 0; k < places; k++) e[4 * 32 * h + k] = bucketEntry(c, (int)s, st, nx, b, kClassBytes * (uint32_t)k);
+    }
   }
   __syncthreads();
 }
 
-// Symbol-log bookkeeping of the symbol path.  kNoError: no failing symbol;
-// kFullChain (in TileStat::errAt): the tile was decoded by the full chain;
-// kOverflow: internal status of a symbol chain whose log ran out of room
-// (never reported: the tile is decoded again by the full chain).  A
-// macroblock header takes at most 125 symbols (mode, reference, partition,
-// four vectors of two class-coded components of up to 15 symbols each,
-// pattern, transform size).
-constexpr int32_t kNoError = 0x7FFFFFFF;
-constexpr int32_t kFullChain = -1;
-constexpr int32_t kOverflow = -100;
-constexpr int kMBHeaderSymbols = 128;
-
-// A tile's rANS decoder (ebiv/rans.go:222-304).  All fields are warp-uniform;
-// the two next stream bytes are prefetched so renormalisation rarely waits.
-// After the first error every symbol decodes as 0.  With kLog every symbol
-// the decoder returns while no error is pending (the failing one included,
-// as 0) is appended to a symbol log, and errAt is the failing one's index.
-template <bool kLog>
-struct ChainT {
+// A tile's rANS decoder as the full chain runs it (ebiv/rans.go:222-304).
+// All fields are warp-uniform; the two next stream bytes are prefetched so
+// renormalisation rarely waits.  After the first error every symbol decodes
+// as 0.
+struct WarpChain {
   const uint8_t* buf;
   int32_t pos;
   uint32_t x0, x1, x2, x3;  // states in use order: x0 decodes the next symbol
   uint32_t b1, b2;          // buf[pos-1], buf[pos-2] when present
   int32_t err;
   const EntropyTables* t;
-  uint8_t* log;   // kLog: the tile's symbol log
-  int32_t n;      // kLog: symbols logged
-  int32_t errAt;  // kLog: index of the failing symbol (kNoError: none)
-  int32_t cap;    // kLog: the log's capacity
-  int32_t lane;   // kLog: the lane that writes the log
 
   __device__ __forceinline__ uint32_t byteAt(int i) const { return i >= 0 ? (uint32_t)__ldg(buf + i) : 0u; }
-  __device__ __forceinline__ int logged(int s) {
-    if (kLog) {
-      if (lane == 0) log[n] = (uint8_t)s;
-      n++;
-    }
-    return s;
-  }
   __device__ __forceinline__ int fail(int e) {
     err = e;
-    if (kLog) errAt = n;
-    return logged(0);
+    return 0;
   }
 
-  // The next symbol of the context whose bucket row starts at word row
-  // (context * 64).
+  // The next symbol of context row / 64.
   __device__ __forceinline__ int symAt(int row) {
     if (err) return 0;
     const uint32_t x = x0;
     const uint32_t slot = x & (kM - 1);
-    const uint32_t e = t->bucket[row + (int)(slot >> 6)];
-    int s = (int)((e >> 25) & 15u);
-    uint32_t start = e & 0xFFFu, freq = (e >> 12) & 0x1FFFu;
-    if (e & (kBImpure | kBUnused)) {
-      if (e & kBUnused) return fail(kErrCorrupt);  // symbol decoded from an unused context
-      while (slot >= start + freq) {
-        const uint32_t w = t->sym[(row >> 2) + (++s)];
-        start = w & 0xFFFFu;
-        freq = w >> 16;
-      }
+    const uint4* e = t->entry + rowOf(row >> 6) / 16 + (slot >> 6) * 4;
+    if (e->z & kEUnused) return fail(kErrCorrupt);  // symbol decoded from an unused context
+    if (e->z & kEImpure) {
+      e = t->entry + e->y;
+      while (slot >= e[1].y) e++;
     }
-    uint32_t xn = freq * (x >> kScaleBits) + slot - start;
+    uint32_t xn = e->x * (x >> kScaleBits) + x - e->y;
     if (xn < kLower) {
       if (pos >= 2 && xn >= (kLower >> 16)) {
         if (xn < (kLower >> 8)) {  // two bytes
@@ -186,16 +158,9 @@ struct ChainT {
     x1 = x2;
     x2 = x3;
     x3 = xn;
-    return logged(s);
+    return (int)((e->w >> kLogShift) & (row < ctxTokenBase << 6 ? 15u : 7u));
   }
   __device__ __forceinline__ int sym(int ctx) { return symAt(ctx << 6); }
-  // Whether the log has room for `need` more symbols; when it has not, the
-  // chain stops with kOverflow.
-  __device__ __forceinline__ bool room(int need) {
-    if (!kLog || n + need <= cap) return true;
-    err = kOverflow;
-    return false;
-  }
   // Initialises the four states from the end of the tile's bytes
   // (ransDecoder.reset, ebiv/rans.go:236-250); false when the stream is too short.
   __device__ __forceinline__ bool reset(const uint8_t* b, uint32_t len, const EntropyTables* tables) {
@@ -203,8 +168,6 @@ struct ChainT {
     pos = (int32_t)len;
     err = 0;
     t = tables;
-    n = 0;
-    errAt = kNoError;
     if (len < (uint32_t)(kStates * 4)) {
       err = kErrCorrupt;
       return false;
@@ -225,58 +188,21 @@ struct ChainT {
   }
 };
 
-// Replays a tile's symbol log from one macroblock's first symbol: the same
-// values, and the same error state at every point, as the chain that wrote
-// the log (a symbol past the failing one is never read: it decodes as 0).
-struct Replay {
-  const uint8_t* log;
-  int32_t k;      // index of the next symbol in the tile's log
-  int32_t errAt;  // index of the failing symbol, or kNoError
-  int32_t end;    // the log's capacity: reads stay inside it
-  int32_t err;
-  __device__ __forceinline__ int symAt(int) {
-    if (err) return 0;
-    if (k >= end) {  // unreachable while replay and chain agree; keeps every read in bounds
-      err = kErrCorrupt;
-      return 0;
-    }
-    const int s = log[k];
-    k++;
-    if (k > errAt) err = kErrCorrupt;
-    return s;
-  }
-  __device__ __forceinline__ int sym(int) { return symAt(0); }
-  __device__ __forceinline__ bool room(int) const { return true; }
-};
-
 // getRawBits / getClassValue / getMVComponent — ebiv/mv.go:75-128.
-template <class S>
-__device__ __forceinline__ uint32_t rawBits(S& d, int n) {
-  uint32_t v = 0;
-  for (int i = 0; i < n; i++) v = v << 1 | (uint32_t)d.sym(ctxBypass);
+__device__ __forceinline__ uint32_t classValue(WarpChain& d, int classCtx) {
+  const int cls = d.sym(classCtx);
+  uint32_t v = (uint32_t)min(cls, 1);
+  for (int i = 1; i < cls; i++) v = v << 1 | (uint32_t)d.sym(ctxBypass);
   return v;
 }
-template <class S>
-__device__ __forceinline__ uint32_t classValue(S& d, int classCtx) {
-  const int cls = d.sym(classCtx);
-  if (cls <= 1) return (uint32_t)cls;
-  return (1u << (cls - 1)) | rawBits(d, cls - 1);
-}
-template <class S>
-__device__ __forceinline__ int mvComponent(S& d, int classCtx) {
-  const uint32_t u = classValue(d, classCtx);
-  return (int)(u >> 1) ^ -(int)(u & 1);
-}
+__device__ __forceinline__ int unzigzag(uint32_t u) { return (int)(u >> 1) ^ -(int)(u & 1); }
+__device__ __forceinline__ int mvComponent(WarpChain& d, int classCtx) { return unzigzag(classValue(d, classCtx)); }
 
-// decodeBlock (ebiv/residual.go:79-126).  With kOut the block's nonzero
-// levels are written as packed entries after a count word (by lane 0);
-// without it only the symbols are decoded (the chain of the symbol path:
-// everything that decides which symbol comes next, nothing else).  row is
-// the bucket row of the block's token contexts at band 0 and previous class
-// 0 (context * 64); the band and previous class add their row offsets.
-// Returns the count.
-template <bool kOut, class S>
-__device__ __forceinline__ int entropyBlock(S& d, int row, int sz, uint32_t* region, int lane) {
+// decodeBlock (ebiv/residual.go:79-126): the block's nonzero levels are
+// written as packed entries after a count word (by lane 0).  row is the entry
+// row of the block's token contexts at band 0 and previous class 0 (context *
+// 64); the band and previous class add their row offsets.  Returns the count.
+__device__ __forceinline__ int entropyBlock(WarpChain& d, int row, int sz, uint32_t* region, int lane) {
   const uint32_t* sb = cScanRow[sz];
   const int total = 16 << (2 * sz);
   int first = -1, last = -1, count = 0;
@@ -310,7 +236,7 @@ __device__ __forceinline__ int entropyBlock(S& d, int row, int sz, uint32_t* reg
       firstMag = mag;
     } else {
       if (d.symAt(ctxSign << 6) == 1) mag = -mag;
-      if (kOut && lane == 0) region[1 + count] = pos | ((uint32_t)mag << 8);
+      if (lane == 0) region[1 + count] = pos | ((uint32_t)mag << 8);
     }
     count++;
     last = i;
@@ -318,9 +244,9 @@ __device__ __forceinline__ int entropyBlock(S& d, int row, int sz, uint32_t* reg
   }
   if (first >= 0) {
     const bool neg = (last - first >= kSDHMinSpan) ? (sumAbs & 1) == 1 : d.symAt(ctxSign << 6) == 1;
-    if (kOut && lane == 0) region[1] = firstPos | ((uint32_t)(neg ? -firstMag : firstMag) << 8);
+    if (lane == 0) region[1] = firstPos | ((uint32_t)(neg ? -firstMag : firstMag) << 8);
   }
-  if (kOut && lane == 0) region[0] = (uint32_t)count;
+  if (lane == 0) region[0] = (uint32_t)count;
   return count;
 }
 
@@ -357,13 +283,6 @@ struct Rec {
     else if (i == 1) mv1 = v;
     else if (i == 2) mv2 = v;
     else mv3 = v;
-  }
-  // One thread stores the whole 48-byte record.
-  __device__ __forceinline__ void storeAll(MBRec* dst) const {
-    uint4* q = reinterpret_cast<uint4*>(dst);
-    q[0] = make_uint4(w0, w1, mv0, mv1);
-    q[1] = make_uint4(mv2, mv3, lm0, lm1);
-    q[2] = make_uint4(lm2, lm3, nz, wm);
   }
   // Lanes 0-2 store the 48-byte record as three 16-byte words.
   __device__ __forceinline__ void store(MBRec* dst, int lane) const {
@@ -404,10 +323,7 @@ struct BlockPlan {
 
 // The block loop of a macroblock.  Returns how many blocks completed before
 // an error; *nzOut gets the nonzero mask (bit k luma block k, 16 Cb, 17 Cr).
-// A logging chain first checks that its log has room for the block's
-// largest possible symbol count (mode, 17 per coefficient, the hidden sign).
-template <bool kOut, class S>
-__device__ __forceinline__ int entropyBlocks(S& d, Rec& r, const BlockPlan& p, uint32_t* coef, int lane,
+__device__ __forceinline__ int entropyBlocks(WarpChain& d, Rec& r, const BlockPlan& p, uint32_t* coef, int lane,
                                              uint32_t* nzOut) {
   const int nEnt = p.nLuma + (p.cb ? 1 : 0) + (p.cr ? 1 : 0);
   const int bw = (16 << (2 * p.tx)) + 1;  // words per luma block region
@@ -421,21 +337,19 @@ __device__ __forceinline__ int entropyBlocks(S& d, Rec& r, const BlockPlan& p, u
     uint32_t bit;
     if (e < p.nLuma) {
       sz = p.tx;
-      if (!d.room(2 + 17 * (16 << (2 * sz)))) break;
       if (p.intra) r.lumaMode(e, (uint32_t)d.sym(ctxLumaMode));
       row = lumaRow;
       region = coef + e * bw;
       bit = 1u << e;
     } else {
       sz = 1;
-      if (!d.room(2 + 17 * 64)) break;
       const bool isCb = p.cb && e == p.nLuma;
       if (isCb && p.intra) r.w1 |= (uint32_t)d.sym(ctxChromaMode) << 8;
       row = (ctxTokenBase + kLumaTokenCtx) << 6;
       region = coef + (isCb ? kCoefCb : kCoefCr);
       bit = isCb ? (1u << 16) : (1u << 17);
     }
-    const int cnt = entropyBlock<kOut>(d, row, sz, region, lane);
+    const int cnt = entropyBlock(d, row, sz, region, lane);
     if (d.err) break;
     if (cnt) nz |= bit;
     done++;
@@ -446,8 +360,7 @@ __device__ __forceinline__ int entropyBlocks(S& d, Rec& r, const BlockPlan& p, u
 
 // Intra macroblock header (decodeLumaMB, ebiv/decode_intra.go:137-150): the
 // transform size; the blocks follow.
-template <class S>
-__device__ __forceinline__ void intraHeader(S& d, Rec& r, BlockPlan* p) {
+__device__ __forceinline__ void intraHeader(WarpChain& d, Rec& r, BlockPlan* p) {
   int tx = d.sym(ctxTxSize);
   if (tx >= 3) tx = 0;  // alphabet size 3: unreachable
   r.w0 = kRecIntra;
@@ -463,8 +376,7 @@ __device__ __forceinline__ void intraHeader(S& d, Rec& r, BlockPlan* p) {
 // (x, y as int16) in the record; predictVectors turns them into vectors
 // (no context depends on a vector, so the chain never needs them).  Returns
 // 1 when the blocks of *p follow, 0 when the macroblock ends here (an error).
-template <class S>
-__device__ __forceinline__ int interHeader(S& d, Rec& r, int mode, BlockPlan* p, bool* intra) {
+__device__ __forceinline__ int interHeader(WarpChain& d, Rec& r, int mode, BlockPlan* p, bool* intra) {
   if (mode == mbIntra) {
     *intra = true;
     intraHeader(d, r, p);
@@ -634,31 +546,20 @@ __device__ void predictVectors(const FrameDesc* fp, int tile, int done, WarpRows
 constexpr int kEntropyWarps = kEntropyTilesPerJob;
 
 // One macroblock's grammar (decodeInterMB, ebiv/decode_inter.go:8-62;
-// decodeLumaMB / decodeChromaMB, ebiv/decode_intra.go:137-187).  With kOut
-// the record and the coefficient regions are written: by lanes 0-2 of a
-// warp that runs the macroblock together, or, with kThread, all by the one
-// thread that runs it.  Returns 1 when the macroblock is intra and written
-// (an entry of the tile's intra list).
-template <bool kOut, bool kThread, class S>
-__device__ __forceinline__ int decodeMB(S& d, int inter, MBRec* rec, uint32_t* coef, int lane) {
+// decodeLumaMB / decodeChromaMB, ebiv/decode_intra.go:137-187), run by a warp
+// together; the record is written by lanes 0-2 and the coefficient regions by
+// lane 0.  Returns 1 when the macroblock is intra and written (an entry of
+// the tile's intra list).
+__device__ __forceinline__ int decodeMB(WarpChain& d, int inter, MBRec* rec, uint32_t* coef, int lane) {
   int mode = 0;
   if (inter) {
     mode = d.sym(ctxMBMode);
     if (mode == mbSkip) {
       // Skip macroblock (most of an inter frame): a fixed record whose
       // vector predictVectors fills in; nothing else to decode.
-      if (kOut) {
-        const uint4 a = make_uint4(kRecSkip, 0u, 0u, 0u), z = make_uint4(0u, 0u, 0u, 0u),
-                    c = make_uint4(0u, 0u, 0u, kWriteAll);
-        uint4* q = reinterpret_cast<uint4*>(rec);
-        if (kThread) {
-          q[0] = a;
-          q[1] = z;
-          q[2] = c;
-        } else if (lane < 3) {
-          q[lane] = lane == 0 ? a : (lane == 1 ? z : c);
-        }
-      }
+      const uint4 a = make_uint4(kRecSkip, 0u, 0u, 0u), z = make_uint4(0u, 0u, 0u, 0u),
+                  c = make_uint4(0u, 0u, 0u, kWriteAll);
+      if (lane < 3) reinterpret_cast<uint4*>(rec)[lane] = lane == 0 ? a : (lane == 1 ? z : c);
       return 0;
     }
   }
@@ -676,15 +577,12 @@ __device__ __forceinline__ int decodeMB(S& d, int inter, MBRec* rec, uint32_t* c
   }
   if (blocks) {
     uint32_t nz;
-    const int nd = entropyBlocks<kOut>(d, r, p, coef, kThread ? 0 : lane, &nz);
+    const int nd = entropyBlocks(d, r, p, coef, lane, &nz);
     r.nz = nz;
     w = writeMask(p, nd);
   }
   r.wm = w;
-  if (kOut) {
-    if (kThread) r.storeAll(rec);
-    else r.store(rec, lane);
-  }
+  r.store(rec, lane);
   return intra && w ? 1 : 0;
 }
 
@@ -703,14 +601,13 @@ __device__ __noinline__ int fullChain(const FrameDesc* fp, int tile, const Entro
   uint32_t* const intraList = fp->intraList + tr.mbBase;
   const int x0 = tr.mbX0, x1 = tr.mbX1, y0 = tr.mbY0, y1 = tr.mbY1;
   const int tw = x1 - x0, total = tw * (y1 - y0);
-  ChainT<false> d;
+  WarpChain d;
   d.reset(fp->pkt + tr.offset, tr.length, &sT);
-  d.lane = lane;
   int done = 0, intraCount = 0;
   for (int mby = y0; mby < y1 && !d.err; mby++) {
     for (int mbx = x0; mbx < x1; mbx++) {
       const int idx = mby * mbCols + mbx;
-      if (decodeMB<true, false>(d, inter, recs + idx, coefBase + (size_t)idx * kCoefPerMB, lane)) {
+      if (decodeMB(d, inter, recs + idx, coefBase + (size_t)idx * kCoefPerMB, lane)) {
         if (lane == 0) intraList[intraCount] = (uint32_t)idx;
         intraCount++;
       }
@@ -729,44 +626,38 @@ __device__ __noinline__ int fullChain(const FrameDesc* fp, int tile, const Entro
     ts.err = d.err;
     ts.intraCount = intraCount;
     ts.done = done;
-    ts.errAt = kFullChain;
+    ts.fullChain = 1;
     fp->tileStat[tile] = ts;
     if (d.err) atomicExch(fp->status, kErrCorrupt);
   }
   return done;
 }
 
-// The symbol chain of a tile, by one warp: only the rANS decoder and the
-// grammar decisions that pick the next context, every symbol appended to
-// the tile's log and each macroblock's first symbol index recorded; kParse
-// rebuilds the records from the log in parallel.  Returns false when the
-// log would overflow (the caller then runs fullChain).
-__device__ __forceinline__ bool symbolChain(const FrameDesc* fp, int tile, const EntropyTables& sT, int lane) {
-  const int inter = fp->inter;
+// A tile's log and its size in entries: kSymPerMB bytes per macroblock, and
+// for the frame's first tiles room for a macroblock more (the chain reserves
+// that much before each, so that a tile of few macroblocks can use all of its
+// own).
+__device__ __forceinline__ uint16_t* tileLog(const FrameDesc* fp, const TileRange& tr, int tile, int* entries) {
+  static_assert(kSpareLogBytes >= 2 * kMBEntries && kSpareLogBytes % 16 == 0, "spare room of a tile's log");
+  const int total = (tr.mbX1 - tr.mbX0) * (tr.mbY1 - tr.mbY0);
+  *entries = (total * kSymPerMB + (tile < kSpareLogTiles ? kSpareLogBytes : 0)) / 2;
+  return reinterpret_cast<uint16_t*>(fp->symLog + (size_t)tr.mbBase * kSymPerMB +
+                                     (size_t)min(tile, kSpareLogTiles) * kSpareLogBytes);
+}
+
+// The symbol chain of a tile, by one thread (Chain); false when it leaves the
+// tile to the full chain.
+__device__ __forceinline__ bool symbolChain(const FrameDesc* fp, int tile, const EntropyTables& sT) {
   const TileRange tr = fp->tiles[tile];
-  const int tw = tr.mbX1 - tr.mbX0, total = tw * (tr.mbY1 - tr.mbY0);
-  uint32_t* const mbOff = fp->symOff + tr.mbBase;
-  ChainT<true> d;
-  d.reset(fp->pkt + tr.offset, tr.length, &sT);
-  d.lane = lane;
-  d.log = fp->symLog + (size_t)tr.mbBase * fp->symPerMB;
-  d.cap = total * fp->symPerMB;
-  if (d.err) d.errAt = 0;  // too short to initialise: the tile fails at once
-  int done = 0;
-  for (int k = 0; k < total && !d.err; k++) {
-    if (lane == 0) mbOff[k] = (uint32_t)d.n;
-    if (!d.room(kMBHeaderSymbols)) break;
-    decodeMB<false, false>(d, inter, nullptr, nullptr, lane);
-    done++;
-  }
-  if (d.err == kOverflow) return false;
-  if (lane == 0) {
-    TileStat* ts = fp->tileStat + tile;
-    ts->err = d.err;
-    ts->done = done;
-    ts->errAt = d.errAt;
-    if (d.err) atomicExch(fp->status, kErrCorrupt);
-  }
+  const int total = (tr.mbX1 - tr.mbX0) * (tr.mbY1 - tr.mbY0);
+  int cap;
+  uint16_t* const log = tileLog(fp, tr, tile, &cap);
+  Chain d;
+  if (!d.run(fp->pkt + tr.offset, tr.length, sT, fp->inter, total, log, cap, fp->symOff + tr.mbBase)) return false;
+  TileStat* ts = fp->tileStat + tile;
+  ts->err = 0;
+  ts->done = total;
+  ts->fullChain = 0;
   return true;
 }
 
@@ -777,9 +668,10 @@ __device__ __forceinline__ bool symbolChain(const FrameDesc* fp, int tile, const
 // persistent: each CTA takes jobs (longest first, as listed) until none are
 // left, so a round with more jobs than resident CTAs has no second-wave
 // tail; without one, CTA b runs job b.
-__global__ void __launch_bounds__(32 * kEntropyWarps, 4) kEntropy(const FrameDesc* frames, const int4* jobs, int njobs,
+__global__ void __launch_bounds__(32 * kEntropyWarps, 2) kEntropy(const FrameDesc* frames, const int4* jobs, int njobs,
                                                                    int* next) {
-  __shared__ EntropyTables sT;
+  extern __shared__ __align__(16) uint8_t sTables[];
+  EntropyTables& sT = *reinterpret_cast<EntropyTables*>(sTables);
   __shared__ int sJob;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (;;) {
@@ -792,7 +684,16 @@ __global__ void __launch_bounds__(32 * kEntropyWarps, 4) kEntropy(const FrameDes
     buildTables(sT, *fp->tables, threadIdx.x, blockDim.x);
     if (warp < job.z) {
       const int tile = job.y + warp;
-      if (!fp->symLog || !symbolChain(fp, tile, sT, lane)) fullChain(fp, tile, sT, lane);
+      bool done = false;
+      if (fp->symLog) {
+        const TileRange tr = fp->tiles[tile];
+        const int mbs = (tr.mbX1 - tr.mbX0) * (tr.mbY1 - tr.mbY0);
+        for (int k = lane; k < mbs; k += 32) fp->symOff[tr.mbBase + k] = kSkipOffset;
+        __syncwarp();
+        if (lane == 0) done = symbolChain(fp, tile, sT);
+        done = __shfl_sync(kFull, done ? 1 : 0, 0) != 0;
+      }
+      if (!done) fullChain(fp, tile, sT, lane);
     }
     if (!next) return;
     __syncthreads();  // every warp is done with sT and sJob before the next job
@@ -800,85 +701,199 @@ __global__ void __launch_bounds__(32 * kEntropyWarps, 4) kEntropy(const FrameDes
 }
 
 // Rebuilds the records of the symbol-path tiles from their logs, one warp
-// per macroblock over every macroblock of the launch's tiles (grid.y: job *
-// kEntropyTilesPerJob + tile within the job; grid.x * kParseWarps: the
-// macroblock's raster index within its tile).  The warp first copies a
-// window of the tile's log from the macroblock's first symbol into shared
-// memory (aligned 16-byte loads), then replays the macroblock's grammar
-// (decodeMB, the warp's lanes writing the record and the coefficient
-// regions) reading the window, and past it the log in global memory.  A flag
-// per macroblock marks the written intra ones for kTileFinish.
+// per macroblock over every macroblock of the launch's tiles (grid.x: job *
+// kEntropyTilesPerJob + tile within the job; grid.y * kParseWarps: the
+// macroblock's raster index within its tile).  A skip macroblock's record is
+// fixed; of another one the whole warp reads the header, and then each lane
+// one log entry at a time of its blocks: the entries name their kind, so a
+// lane finds its block, its position and its place among the block's levels
+// by counting the ends and tokens before it.  A flag per macroblock marks the
+// intra ones for kTileFinish.
 constexpr int kParseWarps = 8;
-constexpr int kParseWindow = 512;  // bytes of log per warp in shared memory
 
-struct WindowReplay {
-  const uint8_t* win;  // shared: log bytes [w0, w0 + wlen)
-  const uint8_t* log;  // global: the tile's log
-  int32_t w0, wlen, k, errAt, end, err;
-  __device__ __forceinline__ int symAt(int) {
-    if (err) return 0;
-    if (k >= end) {  // unreachable while replay and chain agree; keeps every read in bounds
-      err = kErrCorrupt;
-      return 0;
-    }
-    const int r = k - w0;
-    const int s = r < wlen ? win[r] : log[k];
-    k++;
-    if (k > errAt) err = kErrCorrupt;
-    return s;
-  }
-  __device__ __forceinline__ int sym(int) { return symAt(0); }
-  __device__ __forceinline__ bool room(int) const { return true; }
+struct ParseBlocks {
+  uint32_t nz;     // blocks with levels (bit k luma block k, 16 Cb, 17 Cr)
+  uint32_t cmode;  // the chroma intra mode
 };
 
+// The blocks of plan p whose entries start at entry `from` of the 32 entries
+// at log index `off` (lane's entry of them: v); nothing at or past `end` is
+// read.  Levels go to coef, luma modes to lmode (shared memory).
+__device__ __forceinline__ ParseBlocks parseBlocks(const uint16_t* log, int off, int end, int from, uint32_t v,
+                                                   const BlockPlan& p, uint32_t* coef, uint8_t* lmode, int lane) {
+  ParseBlocks out = {0u, 0u};
+  const int blocks = p.nLuma + (p.cb ? 1 : 0) + (p.cr ? 1 : 0);
+  const int perBlock = (16 << (2 * p.tx)) + 1;  // words per luma block region
+  const unsigned before = (1u << lane) - 1u;
+  auto entry = [&](int i) { return i < end ? (uint32_t)log[i] : 0u; };
+  // The block that is open at the start of a pass: its tokens and nonzero ones
+  // so far, the first one's position and magnitude, the last one's position
+  // and the parity of the magnitudes.
+  int done = 0, openTokens = 0, openCount = 0, openFirst = 0, openMag = 0, openLast = 0, openOdd = 0;
+  while (done < blocks) {
+    const uint32_t kind = v & kLogKind;
+    const int sym = (int)((v >> kLogShift) & 7u);
+    const bool isEnd = kind == kLogToken && sym == tEOB;
+    // The entries of this pass that count: from `from` up to the last block's end.
+    unsigned valid = ~((1u << from) - 1u);
+    unsigned ends = __ballot_sync(kFull, isEnd) & valid;
+    const unsigned last = __ballot_sync(kFull, ((ends >> lane) & 1u) && done + __popc(ends & before) == blocks - 1);
+    if (last) {
+      valid &= last | (last - 1u);
+      ends &= valid;
+    }
+    const unsigned tokens = __ballot_sync(kFull, kind == kLogToken && !isEnd) & valid;
+    const unsigned levels = __ballot_sync(kFull, kind == kLogToken && (v & kLogNonzero) != 0) & valid;
+    const bool isLevel = (levels >> lane) & 1u, ends_here = (ends >> lane) & 1u;
+    // The entry after this one: a token's sign, the last sign of an end, or an
+    // escape's value, whose second half and sign follow.
+    const int at = off + lane;
+    uint32_t next = isLevel || ends_here ? entry(at + 1) : 0u;
+    int mag = sym;
+    if (isLevel && sym == tEscape) {
+      mag = 5 + (int)((next & 0xFF00u) | entry(at + 2) >> kLogShift);
+      next = entry(at + 3);
+    }
+    const bool minus = (next >> kLogShift) & 1u;
+    const unsigned odd = __ballot_sync(kFull, isLevel && (mag & 1));
+    // This lane's block and, of the entries before the lane in this pass,
+    // those of the block.
+    const unsigned endsBefore = ends & before;
+    const int blk = done + __popc(endsBefore);
+    const bool opened = endsBefore == 0;  // the block may have begun in an earlier pass
+    const unsigned mine = opened ? before : before & ~((2u << (31 - __clz(endsBefore))) - 1u);
+    const int pos = __popc(tokens & mine) + (opened ? openTokens : 0);
+    const unsigned mineLevels = levels & mine;
+    const int index = __popc(mineLevels) + (opened ? openCount : 0);
+    const int firstLane = (__ffs(mineLevels) - 1) & 31, lastLane = (31 - __clz(mineLevels)) & 31;
+    int firstPos = __shfl_sync(kFull, pos, firstLane), firstMag = __shfl_sync(kFull, mag, firstLane);
+    int lastPos = __shfl_sync(kFull, pos, lastLane);
+    if (opened && openCount) {
+      firstPos = openFirst;
+      firstMag = openMag;
+      if (!mineLevels) lastPos = openLast;
+    }
+    const bool isLuma = blk < p.nLuma;
+    const bool isCb = p.cb && blk == p.nLuma;
+    uint32_t* const region = coef + (isLuma ? blk * perBlock : (isCb ? kCoefCb : kCoefCr));
+    const uint8_t* const scan = gScan[isLuma ? p.tx : 1];
+    uint32_t bit = 0;
+    if (isLevel) {
+      if (index > 0) region[1 + index] = (uint32_t)scan[pos] | (uint32_t)(minus ? -mag : mag) << 8;
+    } else if (ends_here) {
+      region[0] = (uint32_t)index;
+      if (index > 0) {
+        const bool hidden = lastPos - firstPos >= kSDHMinSpan;
+        const bool neg = hidden ? ((__popc(odd & mine) + (opened ? openOdd : 0)) & 1) != 0 : minus;
+        region[1] = (uint32_t)scan[firstPos] | (uint32_t)(neg ? -firstMag : firstMag) << 8;
+        bit = isLuma ? 1u << blk : (isCb ? 1u << 16 : 1u << 17);
+      }
+    } else if (kind == kLogMode && ((valid >> lane) & 1u) && isLuma) {
+      lmode[blk] = (uint8_t)((v >> kLogShift) & 15u);
+    }
+    const unsigned modes = __ballot_sync(kFull, kind == kLogMode && !isLuma) & valid;
+    if (modes) out.cmode = (__shfl_sync(kFull, v, __ffs(modes) - 1) >> kLogShift) & 15u;
+    out.nz |= __reduce_or_sync(kFull, bit);
+    done += __popc(ends);
+    if (last) break;
+    // What is open after this pass.
+    unsigned tail = valid;
+    if (ends) {
+      tail &= ~((2u << (31 - __clz(ends))) - 1u);
+      openTokens = openCount = openOdd = 0;
+    }
+    const unsigned tailLevels = levels & tail;
+    if (tailLevels) {
+      const int f = __shfl_sync(kFull, pos, __ffs(tailLevels) - 1), m = __shfl_sync(kFull, mag, __ffs(tailLevels) - 1);
+      if (!openCount) {
+        openFirst = f;
+        openMag = m;
+      }
+      openLast = __shfl_sync(kFull, pos, 31 - __clz(tailLevels));
+      openCount += __popc(tailLevels);
+      openOdd ^= __popc(odd & tail) & 1;
+    }
+    openTokens += __popc(tokens & tail);
+    off += 32;
+    from = 0;
+    if (off >= end) break;  // unreachable: the log holds every block's end
+    v = entry(off + lane);
+  }
+  return out;
+}
+
 __global__ void __launch_bounds__(32 * kParseWarps) kParseMB(const FrameDesc* frames, const int4* jobs, int njobs) {
-  __shared__ __align__(16) uint8_t sWin[kParseWarps][kParseWindow];
+  __shared__ __align__(16) uint8_t sMode[kParseWarps][16];
   const int jb = (int)blockIdx.x / kEntropyTilesPerJob, tj = (int)blockIdx.x % kEntropyTilesPerJob;
   if (jb >= njobs) return;
   const int4 job = jobs[jb];
   if (tj >= job.z) return;
   const FrameDesc* fp = frames + job.x;
   const int tile = job.y + tj;
-  const TileStat st = fp->tileStat[tile];
-  if (st.errAt == kFullChain) return;
+  if (fp->tileStat[tile].fullChain) return;
   const TileRange tr = fp->tiles[tile];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tw = tr.mbX1 - tr.mbX0, total = tw * (tr.mbY1 - tr.mbY0);
   const int k = (int)blockIdx.y * kParseWarps + warp;
   if (k >= total) return;
   const int idx = (tr.mbY0 + k / tw) * fp->mbCols + tr.mbX0 + k % tw;
-  MBRec* const rec = fp->mbrec + idx;
+  uint4* const words = reinterpret_cast<uint4*>(fp->mbrec + idx);
   uint8_t* const flags = reinterpret_cast<uint8_t*>(fp->lvgrid) + tr.mbBase;
-  if (k >= st.done) {  // never reached: left untouched by reconstruction
-    if (lane == 0) {
-      rec->mode = kRecNone;
-      rec->wmask = 0;
-      flags[k] = 0;
-    }
+  const uint32_t off = fp->symOff[tr.mbBase + k];
+  if (off == kSkipOffset) {
+    if (lane < 3) words[lane] = make_uint4(lane ? 0u : (uint32_t)kRecSkip, 0u, 0u, lane == 2 ? kWriteAll : 0u);
+    if (lane == 0) flags[k] = 0;
     return;
   }
-  const uint8_t* const log = fp->symLog + (size_t)tr.mbBase * fp->symPerMB;
-  const int end = total * fp->symPerMB;
-  const int first = (int)fp->symOff[tr.mbBase + k];
-  // The window: the aligned 16-byte blocks from the one holding the first
-  // symbol, clipped to the tile's log.
-  const int w0 = first & ~15;
-  const int wlen = max(0, min(kParseWindow, (end & ~15) - w0));  // whole 16-byte blocks only
-  uint8_t* const win = sWin[warp];
-  for (int o = lane * 16; o < wlen; o += 32 * 16)
-    *reinterpret_cast<uint4*>(win + o) = *reinterpret_cast<const uint4*>(log + w0 + o);
+  int end;
+  const uint16_t* const log = tileLog(fp, tr, tile, &end);
+  const uint32_t v = (int)off + lane < end ? (uint32_t)log[off + lane] : 0u;
+  int n = 0;
+  auto next = [&]() -> uint32_t { return (__shfl_sync(kFull, v, n++) >> kLogShift) & 255u; };
+  auto value = [&]() -> uint32_t {
+    const uint32_t high = next();
+    return high << 8 | next();
+  };
+  const int mode = fp->inter ? (int)next() : (int)mbIntra;
+  uint32_t w0 = kRecIntra, cbp = kNumCBP - 1;
+  uint32_t mv[4] = {0u, 0u, 0u, 0u};
+  if (mode != mbIntra) {
+    const uint32_t ref = next(), part = next();
+    const int np = part == partWhole ? 1 : (part == part8x8 ? 4 : 2);
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      if (i < np) {
+        const int x = unzigzag(value()), y = unzigzag(value());
+        mv[i] = packMV(x, y);
+      }
+    cbp = next();
+    w0 = kRecInter | ref << 8 | part << 16 | cbp << 24;
+  }
+  BlockPlan p;
+  p.tx = 0;
+  p.nLuma = 0;
+  p.intra = mode == mbIntra;
+  p.cb = (cbp & cbpCb) != 0;
+  p.cr = (cbp & cbpCr) != 0;
+  if (cbp & cbpLuma) {
+    p.tx = (int)min(next(), 2u);
+    p.nLuma = 16 >> (2 * p.tx);
+  }
+  uint8_t* const lmode = sMode[warp];
+  if (lane < 4) reinterpret_cast<uint32_t*>(lmode)[lane] = 0;
   __syncwarp();
-  WindowReplay r;
-  r.win = win;
-  r.log = log;
-  r.w0 = w0;
-  r.wlen = wlen;
-  r.k = first;
-  r.errAt = st.errAt;
-  r.end = end;
-  r.err = r.k > r.errAt ? kErrCorrupt : 0;
-  const int f = decodeMB<true, false>(r, fp->inter, rec, fp->coef + (size_t)idx * kCoefPerMB, lane);
-  if (lane == 0) flags[k] = (uint8_t)f;
+  const ParseBlocks b = parseBlocks(log, (int)off, end, n, v, p, fp->coef + (size_t)idx * kCoefPerMB, lmode, lane);
+  __syncwarp();
+  if (lane < 3) {
+    // Every block is there, so all of the macroblock is written (of an intra
+    // one, the blocks that its transform size has).
+    const uint32_t wm = p.intra ? ((1u << p.nLuma) - 1u) | 3u << 16 : kWriteAll;
+    const uint32_t* lm = reinterpret_cast<const uint32_t*>(lmode);
+    words[lane] = lane == 0   ? make_uint4(w0, (uint32_t)p.tx | b.cmode << 8, mv[0], mv[1])
+                  : lane == 1 ? make_uint4(mv[2], mv[3], lm[0], lm[1])
+                              : make_uint4(lm[2], lm[3], b.nz, wm);
+  }
+  if (lane == 0) flags[k] = p.intra ? 1 : 0;
 }
 
 // After kParseMB: per tile (one CTA per tile of a job) the written intra
@@ -900,7 +915,7 @@ __global__ void __launch_bounds__(kParseThreads) kTileFinish(const FrameDesc* fr
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int mbCols = fp->mbCols, tw = tr.mbX1 - tr.mbX0;
   const int done = st.done;
-  if (st.errAt != kFullChain) {
+  if (!st.fullChain) {
     const uint8_t* const flags = reinterpret_cast<const uint8_t*>(fp->lvgrid) + tr.mbBase;
     int base = 0;
     for (int k0 = 0; k0 < done; k0 += kParseThreads) {
@@ -1850,14 +1865,17 @@ __global__ void __launch_bounds__(32 * W, 16 / W)
 // ---------------------------------------------------------------------------
 int uploadCodingTables(const int* scan4, const int* scan8, const int* scan16, const int32_t* dct) {
   uint32_t s[3][257];
+  uint8_t pos[3][256] = {};
   std::memset(s, 0, sizeof(s));
   const int* scans[3] = {scan4, scan8, scan16};
   for (int k = 0; k < 3; k++)
     for (int i = 0; i < (16 << (2 * k)); i++) {
       const int band = bandOf(i);
       s[k][i] = (uint32_t)scans[k][i] | ((uint32_t)(band * kNumPrevClass * 64) << 8);
+      pos[k][i] = (uint8_t)scans[k][i];
     }
   if (cudaMemcpyToSymbol(dev::cScanRow, s, sizeof(s)) != cudaSuccess) return kErrDevice;
+  if (cudaMemcpyToSymbol(dev::gScan, pos, sizeof(pos)) != cudaSuccess) return kErrDevice;
   if (cudaMemcpyToSymbol(dev::gDct, dct, sizeof(int32_t) * 3 * 256) != cudaSuccess) return kErrDevice;
   return kOK;
 }
@@ -1866,20 +1884,23 @@ int uploadCodingTables(const int* scan4, const int* scan8, const int* scan16, co
 // the device holds at once), or null for one CTA per job.
 void launchEntropy(const FrameDesc* frames, const int4* jobs, int njobs, int* next, int maxTileMBs, cudaStream_t s) {
   if (njobs <= 0) return;
-  static int resident[64] = {0};
+  constexpr int kTables = (int)sizeof(dev::EntropyTables);
+  // Per device, once: the shared-memory limit and the CTAs it holds at once.
+  static std::atomic<int> resident[64];
   int dev = 0;
   cudaGetDevice(&dev);
-  int grid = njobs;
-  if (next && dev >= 0 && dev < 64) {
-    if (!resident[dev]) {
-      int perSM = 0, sms = 0;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, dev::kEntropy, 32 * dev::kEntropyWarps, 0);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      resident[dev] = std::max(1, perSM * sms);
-    }
-    grid = std::min(njobs, resident[dev]);
+  const bool known = dev >= 0 && dev < 64;
+  int held = known ? resident[dev].load(std::memory_order_acquire) : 0;
+  if (!held) {
+    int perSM = 0, sms = 0;
+    cudaFuncSetAttribute(dev::kEntropy, cudaFuncAttributeMaxDynamicSharedMemorySize, kTables);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, dev::kEntropy, 32 * dev::kEntropyWarps, kTables);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    held = std::max(1, perSM * sms);
+    if (known) resident[dev].store(held, std::memory_order_release);
   }
-  dev::kEntropy<<<grid, 32 * dev::kEntropyWarps, 0, s>>>(frames, jobs, njobs, next);
+  const int grid = next ? std::min(njobs, held) : njobs;
+  dev::kEntropy<<<grid, 32 * dev::kEntropyWarps, kTables, s>>>(frames, jobs, njobs, next);
   dev::kParseMB<<<dim3(njobs * kEntropyTilesPerJob, (maxTileMBs + dev::kParseWarps - 1) / dev::kParseWarps),
                   32 * dev::kParseWarps, 0, s>>>(frames, jobs, njobs);
   dev::kTileFinish<<<dim3(njobs, kEntropyTilesPerJob), dev::kParseThreads, 0, s>>>(frames, jobs, njobs);

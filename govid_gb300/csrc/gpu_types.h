@@ -50,16 +50,22 @@ constexpr int kEntropyTilesPerJob = 4;
 
 // Bytes of symbol log per macroblock in a decode slot (the entropy stage's
 // symbol path; a tile whose symbols do not fit takes the full chain, which
-// decodes it a second time).  Key frames coded at q18 average about 80
-// symbols per macroblock and more in textured areas, and the chain also
-// reserves room for a whole block before decoding it, so the log holds 192.
-constexpr int kSymPerMB = 192;
+// decodes it a second time).  Key frames coded at q18 average about 125
+// symbols of two bytes per macroblock, small textured ones at q22 185, and the
+// chain also reserves room for a whole block before decoding it, so the log
+// holds 256 symbols.
+constexpr int kSymPerMB = 512;
+// The first tiles of a frame have room for one more macroblock's most symbols
+// each (a frame of more tiles is cut into tiles of many macroblocks, or is
+// decoded by the full chain).
+constexpr int kSpareLogTiles = 64, kSpareLogBytes = 3232;
+constexpr size_t symLogBytes(size_t mbs) { return mbs * kSymPerMB + (size_t)kSpareLogTiles * kSpareLogBytes; }
 
 struct TileStat {
   int32_t err;         // 0 or an ebiv status
   int32_t intraCount;  // intra macroblocks reconstructed in this tile
   int32_t done;        // macroblocks the tile's chain reached (raster order)
-  int32_t errAt;       // symbol path: log index of the failing symbol (or none); -1: full chain
+  int32_t fullChain;   // 1: the full chain decoded the tile (its records and intra list are complete)
 };
 
 // Intra list entries hold the frame macroblock index in bits 0-17.
@@ -104,13 +110,10 @@ struct FrameDesc {
   int32_t pad2;
   uint8_t* dep;
   // Symbol path of the entropy stage (null symLog: every tile takes the full
-  // chain): a log of symPerMB bytes per macroblock, tile t's at
-  // tiles[t].mbBase * symPerMB, and per macroblock the index of its first
-  // symbol in its tile's log (at mbBase + raster index within the tile).
+  // chain): the tiles' logs (symLogBytes), and per macroblock the index of its
+  // first symbol in its tile's log (at mbBase + raster index within the tile).
   uint8_t* symLog;
   uint32_t* symOff;
-  int32_t symPerMB;
-  int32_t pad3;
 };
 
 }  // namespace ebiv
