@@ -53,7 +53,8 @@ namespace dev {
 //   y  start
 //   z  kEAdvance when the next symbol's position in the block is the next one
 //      (tokens, signs, modes), else 0; or, in bit 31, kEStop with the reason:
-//      kEEnd (end of block, escape, last sign, a mode that is not skip),
+//      kEEnd (end of block, last sign and transform size, these with kEBlock,
+//      escape, a mode that is not skip),
 //      kEImpure (a later symbol starts inside the bucket; y is the index, in
 //      entries from the first, of the symbol's own one, from where resolve()
 //      goes on, and x the class of a sign's row) or kEUnused (an unused
@@ -61,7 +62,7 @@ namespace dev {
 //   w  the log entry (bits 0-15; a nonzero token has bit 2 set and the class
 //      it leaves in bits 4-5), and kENonzero for a token of magnitude one to
 //      four
-constexpr uint32_t kEStop = 1u << 31, kEEnd = 1u << 30, kEImpure = 1u << 29, kEUnused = 1u << 28;
+constexpr uint32_t kEStop = 1u << 31, kEEnd = 1u << 30, kEImpure = 1u << 29, kEUnused = 1u << 28, kEBlock = 1u << 27;
 constexpr uint32_t kGroupBytes = 4096, kClassBytes = 16, kBucketMask = 0xFC0, kClassMask = 0x30;
 constexpr uint32_t kGroupMask = 0x1F000;                         // the group in a row
 constexpr uint32_t kERest = 1u << 8;                             // Chain::z: the edge is not the block's end
@@ -115,18 +116,19 @@ constexpr int kMBEntries = 5 + 8 * 2 + 4 * 384 + 18 * 3 + 4;
 EBIV_DEV uint4 symbolEntry(int c, int s, uint32_t st, uint32_t freq, uint32_t cls) {
   uint32_t z = 0, w = (uint32_t)s << kLogShift;
   if (c >= ctxTokenBase) {
-    z = s < tEscape ? kEAdvance : kEStop | kEEnd;
+    z = s < tEscape ? kEAdvance : kEStop | kEEnd | (s == tEOB ? kEBlock : 0u);
     if (s >= tOne && s <= tFour) w |= kENonzero;
     if (s >= tOne && s <= tEscape) w |= kLogNonzero | (s == tOne ? kClassBytes : 2 * kClassBytes);
   } else if (c == ctxSign) {
     const bool last = cls == kClassMask;
-    z = last ? kEStop | kEEnd : kEAdvance;
+    z = last ? kEStop | kEEnd | kEBlock : kEAdvance;
     w |= last ? kLogSign : kLogSign | cls;
   } else if (c == ctxLumaMode || c == ctxChromaMode) {
     z = kEAdvance;
     w |= kLogMode;
   } else {
     if (c == ctxMBMode && s != mbSkip) z = kEStop | kEEnd;
+    if (c == ctxTxSize) z = kEStop | kEEnd | kEBlock;
     w |= kLogValue;
   }
   return make_uint4(freq - kM, st, z, w);
@@ -170,25 +172,26 @@ EBIV_DEV uint4 blockEntry(int kind) {
 // branches, and 270 cycles a symbol.  So the symbols of a macroblock's blocks
 // all take the same straight line (tokens()), four of them, one per rANS
 // state, in a loop: the entry's words turn the state of the grammar into the
-// next by masks, the next entry's address is one load and two logic operations
-// away from the last one's, and one test per symbol, behind the next one's
-// load, finds everything else.  The ends of blocks, last signs and buckets
-// with a boundary then go through a stub beside the line and join it again (a
-// stub of one's own for each state, so that no register moves: 175 and 128
-// cycles); escapes, edges and second stream bytes leave it.  Measured: 105
-// cycles a symbol on the line, 125 to 135 with everything (720p key frame of
-// one tile at q18, 448 thousand symbols: 61 ms before, 30 ms), 31 a skip (77
-// before).  Four symbols to a test would be 70 on the line, but what follows
-// an end in its group is lost and undone: 170 with everything.
+// next by masks, the next entry's address is two logic operations away from
+// this one's entry, and one test per symbol finds everything else.  The ends
+// of blocks, last signs, buckets with a boundary and, in a frame of intra
+// macroblocks, the transform sizes then go through a stub beside the line and
+// join it again (one for each state, so that no register moves); escapes,
+// edges and second stream bytes leave it.  Measured: 91 cycles a symbol on the
+// line, 105 to 120 with everything (720p key frame of one tile at q18, 448
+// thousand symbols: 61 ms before, 26 ms), 31 a skip (77 before).  Issuing the
+// next entry's load before the test instead of after it: 107 on the line; four
+// symbols to a test: 70, but what follows an end in its group is lost and
+// undone, 170 with everything.
 struct Chain {
   uint32_t x0, x1, x2, x3;  // states in use order: x0 decodes the next symbol
   // The stream, read backwards: hi and lo are its next words, off the bits of
   // hi that are used, nw the word after lo, wp its address; rem counts the
   // bits left, below 0 when a symbol has taken a byte before the tile's first
-  // one.  Words wholly before that byte are not read.
+  // one.  The words read ahead are up to 15 bytes before that byte, in the
+  // packet: 78 bytes of headers and tables at least precede a tile.
   uint32_t hi, lo, off, nw;
   const uint32_t* wp;
-  const uint32_t* low;
   int32_t rem;
   const EntropyTables* t;
   uint16_t* log;   // the tile's log
@@ -205,8 +208,13 @@ struct Chain {
   // position after the first nonzero token's and before this one (unary, the
   // oldest lost).  far: bit 2 is set once a nonzero token was kSDHMinSpan or
   // more positions after the first.
+  // The macroblocks: mb is the current one, mbOff their offsets, cap the
+  // log's size; intraOnly: no mode in front of a macroblock.
   uint4 kind;
   int32_t left;
+  int32_t mb, cap;
+  bool intraOnly;
+  uint32_t* mbOff;
   uint32_t queue, z, bands, seen, since, far;
 
   EBIV_DEV uint4 entryAt(uint32_t offset) const {
@@ -233,23 +241,20 @@ struct Chain {
   EBIV_DEV void refill() {
 #ifdef __CUDACC__  // without a branch
     asm volatile(
-        "{\n.reg .pred p, q;\n"
+        "{\n.reg .pred p;\n"
         "setp.ge.u32 p, %2, 32;\n"
         "@p add.u32 %2, %2, -32;\n"
         "@p mov.b32 %0, %1;\n"
         "@p mov.b32 %1, %3;\n"
         "@p add.u64 %4, %4, -4;\n"
-        "setp.ge.and.u64 q, %4, %5, p;\n"
-        "@p mov.u32 %3, 0;\n"
-        "@q ld.global.nc.u32 %3, [%4];\n}"
-        : "+r"(hi), "+r"(lo), "+r"(off), "+r"(nw), "+l"(wp)
-        : "l"(low));
+        "@p ld.global.nc.u32 %3, [%4];\n}"
+        : "+r"(hi), "+r"(lo), "+r"(off), "+r"(nw), "+l"(wp));
 #else
     if (off >= 32) {
       off -= 32;
       hi = lo;
       lo = nw;
-      nw = --wp >= low ? __ldg(wp) : 0u;
+      nw = __ldg(--wp);
     }
 #endif
   }
@@ -300,7 +305,7 @@ struct Chain {
       q -= 16;
     }
     const bool last = e.x == kClassMask;  // the last sign's row; else the row's class (0 but for signs)
-    r.z = last ? kEStop | kEEnd : r.z;
+    r.z = last ? kEStop | kEEnd | kEBlock : r.z;
     r.w |= last ? 0u : e.x;
     return r;
   }
@@ -351,21 +356,42 @@ struct Chain {
     left = (int32_t)((queue >> 4) & 15u);
     queue >>= 8;
   }
-  // The grammar after a block's end or its last sign (the symbol of entry e):
-  // the offset of the next symbol, which state xn decodes.
-  EBIV_DEV uint32_t ended(const uint4& e, uint32_t xn) {
-    const bool sign = (e.w & kLogKind) == kLogToken && (seen & kGroupMask) != 0 && !(far & kLogNonzero);
+  // The blocks of an intra macroblock of transform size tx.
+  static EBIV_DEV uint32_t intraQueue(uint32_t tx) {
+    return (tx + 5u) | ((16u >> (2 * tx)) - 1) << 4 | (8u | 4u << 8) << 8;
+  }
+  // After the last block of a kind: the next kind; in a frame of intra
+  // macroblocks only, the next one's transform size and then its blocks (e is
+  // the symbol of log index `at`).
+  EBIV_DEV void endedKind(const uint4& e, int at) {
+    if ((e.w & kLogKind) == kLogValue) {
+      queue = intraQueue(min((e.w >> kLogShift) & 15u, 2u));  // alphabet size 3
+      mbOff[++mb] = (uint32_t)at;
+    } else if (queue == 0) {
+      if (!intraOnly || mb + 1 >= stop || at + 1 + kMBEntries > cap) return;
+      kind = make_uint4(rowOf(ctxTxSize), 0u, 0u, 0u);
+      left = 0;
+      return;
+    }
+    nextKind();
+  }
+  // The grammar after a block's end, its last sign, or a transform size (the
+  // symbol of entry e, of log index `at`): the offset of the next symbol,
+  // which state xn decodes.
+  EBIV_DEV uint32_t ended(const uint4& e, int at, uint32_t xn) {
+    const bool sign = (seen & kGroupMask) != 0 && !(far & kLogNonzero);
     seen = kClassMask;
     since = far = 0;
     left -= sign ? 0 : 1;
-    if (left < 0 && queue != 0) nextKind();
+    if (left < 0) endedKind(e, at);
     z = left < 0 ? 1u << 31 : kind.y;
     bands = kind.z;
     return (sign ? kLastSignRow : kind.x) | (xn & kBucketMask);
   }
 
   // The symbols of a macroblock's blocks (decodeBlock, ebiv/residual.go:79-126),
-  // which `blocks` lists as `queue` does.
+  // which `blocks` lists as `queue` does, and with intraOnly those of the
+  // macroblocks after it while the log has room for the most they can take.
   EBIV_DEV void tokens(uint32_t blocks) {
     queue = blocks;
     nextKind();
@@ -389,29 +415,38 @@ struct Chain {
   take(X, cur, rem);                          \
   small = X - kLower;                         \
   lp[J] = (uint16_t)E.w;
-#define EBIV_SYMBOL(J, X, XN, E, F)                                                           \
-  symbol##J : F = entryAt(nextAt(E, XN));                                                     \
-  if (__builtin_expect((int32_t)(E.z | z | small1) < 0, 0)) goto stub##J;                     \
+#ifdef __CUDACC__  // keeps the symbol's work here, beside the next entry's load
+#define EBIV_PIN(X) asm volatile("" : "+r"(X), "+r"(z), "+r"(bands), "+r"(seen));
+#else
+#define EBIV_PIN(X)
+#endif
+#define EBIV_PLAIN(J, X, XN, E, F)                                                            \
+  go##J : F = entryAt(nextAt(E, XN));                                                         \
   EBIV_UPDATE(J, X, E)                                                                        \
   follow(E);                                                                                  \
-  next##J:
+  EBIV_PIN(X)
+#define EBIV_MORE(E) __builtin_expect((int32_t)(E.z | z | small1) < 0, 0)
 #define EBIV_STUB(J, X, XN, E, F)                                                             \
-  stub##J : if ((int32_t)(z | small1) < 0 || (E.z & kEUnused) != 0 || (E.w & kLogNonzero) != 0) { \
+  if ((int32_t)(E.z << 4 & ~(z | small1)) < 0) { /* kEBlock */                                \
+    EBIV_UPDATE(J, X, E)                                                                      \
+    F = entryAt(ended(E, count() + J, XN));                                                   \
+  } else {                                                                                    \
     n = J;                                                                                    \
-    goto stopped;                                                                             \
-  }                                                                                           \
-  if (E.z & kEImpure) {                                                                       \
+    if ((int32_t)(z | small1) < 0 || !(E.z & kEImpure)) goto stopped;                         \
     E = resolve(E, X);                                                                        \
-    goto symbol##J;                                                                           \
-  }                                                                                           \
-  EBIV_UPDATE(J, X, E)                                                                        \
-  F = entryAt(ended(E, XN));                                                                  \
-  goto next##J;
+    if ((int32_t)E.z < 0) goto stopped;                                                       \
+    goto go##J;                                                                               \
+  }
     for (;;) {
-      EBIV_SYMBOL(0, x0, x1, e, f)
-      EBIV_SYMBOL(1, x1, x2, f, e)
-      EBIV_SYMBOL(2, x2, x3, e, f)
-      EBIV_SYMBOL(3, x3, x0, f, e)
+      if (EBIV_MORE(e)) goto stub0;
+      EBIV_PLAIN(0, x0, x1, e, f)
+      if (EBIV_MORE(f)) goto stub1;
+      EBIV_PLAIN(1, x1, x2, f, e)
+      if (EBIV_MORE(e)) goto stub2;
+      EBIV_PLAIN(2, x2, x3, e, f)
+      if (EBIV_MORE(f)) goto stub3;
+      EBIV_PLAIN(3, x3, x0, f, e)
+    next3:
       lp += 4;
       off += (uint32_t)(had - rem);
       if (rem < 0) return fail();
@@ -419,10 +454,18 @@ struct Chain {
       had = rem;
       cur = __funnelshift_l(lo, hi, off);
       continue;
+    stub0:
       EBIV_STUB(0, x0, x1, e, f)
+      if (!EBIV_MORE(f)) goto go1;
+    stub1:
       EBIV_STUB(1, x1, x2, f, e)
+      if (!EBIV_MORE(e)) goto go2;
+    stub2:
       EBIV_STUB(2, x2, x3, e, f)
+      if (!EBIV_MORE(f)) goto go3;
+    stub3:
       EBIV_STUB(3, x3, x0, f, e)
+      goto next3;
     stopped:
       lp += n;
       off += (uint32_t)(had - rem);
@@ -470,10 +513,15 @@ struct Chain {
           bands = 1u << 12;
         } else {
           put(tEOB << kLogShift);
-          e = entryAt(ended(make_uint4(0u, 0u, 0u, 0u), x0));
+          e = entryAt(ended(make_uint4(0u, 0u, 0u, 0u), count() - 1, x0));
           if (left < 0) return;
         }
-      } else if ((e.z & kEUnused) != 0 || ((e.z & kEEnd) != 0 && (e.w & kLogNonzero) != 0)) {
+      } else if (e.z & kEBlock) {
+        e = symbolOf(e);
+        put(e.w);
+        e = entryAt(ended(e, count() - 1, x0));
+        if (left < 0) return;
+      } else if ((e.z & (kEUnused | kEEnd)) != 0) {
         // A failure, or an escape: its value, then the sign unless it is the
         // first nonzero token.
         e = symbolOf(e);
@@ -492,7 +540,9 @@ struct Chain {
       cur = __funnelshift_l(lo, hi, off);
     }
 #undef EBIV_STUB
-#undef EBIV_SYMBOL
+#undef EBIV_MORE
+#undef EBIV_PLAIN
+#undef EBIV_PIN
 #undef EBIV_UPDATE
   }
 
@@ -537,10 +587,10 @@ struct Chain {
 
   // Initialises the four states from the end of the tile's bytes
   // (ransDecoder.reset, ebiv/rans.go:236-250); false when the stream is too
-  // short, or when a state is below kLower, as no encoder leaves it (a symbol
-  // then takes at most two bytes).  The bytes down to the first aligned word are read one by one, so
-  // no load reaches past the tile; the words below may reach up to three
-  // bytes before it, where the packet's header and tables are.
+  // short, or when a state is below kLower or at 2^31 and above, as no encoder
+  // leaves it (a symbol of one in between takes at most two bytes and leaves
+  // one).  The bytes down to the first aligned word are read one by one, so no
+  // load reaches past the tile.
   EBIV_DEV bool reset(const uint8_t* buf, uint32_t len, const EntropyTables* tables) {
     t = tables;
     if (len < (uint32_t)(kStates * 4)) return false;
@@ -556,17 +606,15 @@ struct Chain {
     x1 = st[1];
     x2 = st[2];
     x3 = st[3];
-    if (min(min(x0, x1), min(x2, x3)) < kLower) return false;
+    if (min(min(x0, x1), min(x2, x3)) < kLower || ((x0 | x1 | x2 | x3) >> 31) != 0) return false;
     rem = 8 * pos;
     const int head = min(pos, (int)((uintptr_t)(buf + pos) & 3));  // bytes above the last aligned word
     hi = 0;
     for (int k = 0; k < head; k++) hi = hi << 8 | (uint32_t)__ldg(buf + --pos);
     off = 32 - 8 * (uint32_t)head;
-    low = reinterpret_cast<const uint32_t*>((uintptr_t)buf & ~(uintptr_t)3);
     wp = reinterpret_cast<const uint32_t*>((uintptr_t)(buf + pos) & ~(uintptr_t)3) - 1;
-    lo = wp >= low ? __ldg(wp) : 0u;
-    wp--;
-    nw = wp >= low ? __ldg(wp) : 0u;
+    lo = __ldg(wp);
+    nw = __ldg(--wp);
     refill();
     return true;
   }
@@ -577,21 +625,23 @@ struct Chain {
   // when the tile is left to the full chain: a symbol failed, or the log would
   // overflow (before a macroblock there must be room for the most entries it
   // can take).
-  EBIV_DEV bool run(const uint8_t* buf, uint32_t len, const EntropyTables& tables, int inter, int total, uint16_t* tileLog,
-                   int cap, uint32_t* mbOff) {
+  EBIV_DEV bool run(const uint8_t* buf, uint32_t len, const EntropyTables& tables, int inter, int total,
+                    uint16_t* tileLog, int entries, uint32_t* offsets) {
     log = lp = tileLog;
+    cap = entries;
+    mbOff = offsets;
     stop = total;
+    intraOnly = !inter;
     if (!reset(buf, len, &tables)) return false;
-    int k = 0;
 #pragma unroll 1
-    for (; k < stop; k++) {
+    for (mb = 0; mb < stop; mb++) {
       uint32_t mode = mbIntra;
       if (inter) {
-        mode = skips(k, &k);
+        mode = skips(mb, &mb);
         if (mode == mbSkip) break;
       }
       if (count() + kMBEntries > cap) return false;
-      mbOff[k] = (uint32_t)count();
+      mbOff[mb] = (uint32_t)count();
       if (inter) put(kLogValue | mode << kLogShift);
       uint32_t cbp = kNumCBP - 1;
       if (mode != mbIntra) {
@@ -606,19 +656,15 @@ struct Chain {
       }
       // The coded blocks in bitstream order: luma, Cb, Cr; an intra one's mode
       // before each luma block and before Cb.
-      const uint32_t intra = mode == mbIntra ? 4u : 0u;
-      uint32_t blocks = 0;
-      int at = 0;
+      uint32_t tx = 0, blocks = 0;
       if (cbp & cbpLuma) {
-        const uint32_t tx = min(sym(ctxTxSize), 2u);  // alphabet size 3
+        tx = min(sym(ctxTxSize), 2u);  // alphabet size 3
         put(kLogValue | tx << kLogShift);
-        blocks = (tx + intra + 1) | ((16u >> (2 * tx)) - 1) << 4;
-        at = 8;
+        blocks = (tx + 1) | ((16u >> (2 * tx)) - 1) << 4;
       }
-      if (intra)
-        blocks |= (8u | 4u << 8) << at;
-      else
-        blocks |= ((cbp & (cbpCb | cbpCr)) == (cbpCb | cbpCr) ? 4u | 1u << 4 : (cbp & (cbpCb | cbpCr) ? 4u : 0u)) << at;
+      const uint32_t chroma = (cbp & cbpCb ? 1u : 0u) + (cbp & cbpCr ? 1u : 0u);
+      if (chroma) blocks |= (4u | (chroma - 1) << 4) << (cbp & cbpLuma ? 8 : 0);
+      if (mode == mbIntra) blocks = intraQueue(tx);
       if (blocks != 0 && stop != 0) tokens(blocks);
     }
     return stop == total;

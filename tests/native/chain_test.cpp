@@ -32,7 +32,7 @@ struct Plain {
   int pos;
   uint32_t x[4];
   int at = 0;
-  bool err = false, low = false;  // a symbol failed; a state started below kLower
+  bool err = false, low = false;  // a symbol failed; a state started out of range
   std::vector<uint16_t> log;
   std::vector<uint32_t> off;
 
@@ -44,7 +44,7 @@ struct Plain {
     for (int i = 3; i >= 0; i--) {
       pos -= 4;
       x[i] = rd32(buf + pos);
-      low = low || x[i] < kLower;
+      low = low || x[i] < kLower || x[i] >> 31;
     }
   }
   int fail() {
