@@ -184,3 +184,11 @@ def test_hostile_wide_residuals_match_oracle(gpu_required, qp, dense):
         res += [(x.frame_index, x.status, b.download(x, w, h)) for x in b.round()]
     res += [(x.frame_index, x.status, b.download(x, w, h)) for x in b.drain()]
     assert sorted((i, s, p) for i, s, p in res) == [(i, 0, want[i][1]) for i in range(len(pkts))]
+
+
+@pytest.mark.parametrize("w,h", [(16, 16), (32, 48), (112, 32), (48, 528), (144, 560), (2048, 32), (2064, 48)])
+def test_vector_prediction_by_tile_shape(gpu_required, w, h):
+    """One tile of an inter clip, its width and height on both sides of what the vector prediction of a tile holds
+    at once: 1, 2, 3, 7, 9, 128 and 129 macroblocks wide, up to 32 rows and more."""
+    cont, _, rec = encode_gen(w, h, 3, ebiv.synth_pan, intra=20, gop=3, tiles=(1, 1))
+    _check(cont, w, h, rec)
