@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <type_traits>
 
 #include "gpu_types.h"
 #include "symbol_chain.h"
@@ -1234,6 +1235,7 @@ struct ReconView {
   const uint8_t* gold[3];
   int strideY, strideC, padW, padH, padCW, padCH, mbCols;
   int32_t qdc, qac;
+  bool words;  // the planes' 4-byte words are aligned
   const MBRec* mbrec;
   uint32_t* coef;
   __device__ __forceinline__ void load(const FrameDesc& f) {
@@ -1244,6 +1246,8 @@ struct ReconView {
     }
     strideY = f.strideY;
     strideC = f.strideC;
+    words = ((reinterpret_cast<uintptr_t>(rec[0]) | reinterpret_cast<uintptr_t>(rec[1]) |
+              reinterpret_cast<uintptr_t>(rec[2]) | (uintptr_t)strideY | (uintptr_t)strideC) & 3) == 0;
     padW = f.padW;
     padH = f.padH;
     padCW = f.padCW;
@@ -1476,113 +1480,155 @@ __global__ void __launch_bounds__(32 * kInterWarps, 6) kInterRecon(const FrameDe
 // Stage B2: intra reconstruction wavefront
 // ---------------------------------------------------------------------------
 
-// Per-warp scratch of the intra stage.  The macroblock being reconstructed
-// lives in a working area in shared memory together with the samples its
-// prediction may read: area row 0 is the row above the macroblock (from one
-// left of it to 31 right of its left edge: above-left corner, above,
-// above-right), column 0 the column to its left; chroma likewise (9 x 9).
-constexpr int kAreaW = 48;
-struct IntraScratch {
-  int32_t ref[2][4 * 16 + 1];  // one reference array per half-warp block
-  int32_t res[384];            // the macroblock's residual (computed by kInterRecon phase 0)
+// Per-warp scratch of the intra stage: the samples that the macroblock's
+// prediction may read, in shared memory.  Samples go four to a word: rows
+// start at x = 0 in column kAreaX, so that words are aligned.
+// Luma: areaY row 0 is the row above the macroblock (from four left of it to
+// 31 right of its left edge), row 1 + y its row y; colY[k] is the column left
+// of x = 4k, top to bottom (colY[0]: of the macroblock's left neighbour).
+// Chroma has one block a plane: the row above and the column to its left.
+constexpr int kAreaX = 16, kAreaW = 48;
+struct __align__(16) IntraScratch {
+  int32_t res[384];  // the macroblock's residual (computed by kInterRecon phase 0)
   uint8_t areaY[17 * kAreaW];
-  uint8_t areaC[2][9 * 16];
+  uint8_t colY[5][16];
+  uint8_t topC[2][32];
+  uint8_t colC[2][16];
 };
 
-// The reference sample array of predictIntra after substituteRefs, in
-// closed form: ref[0..2n-1] left column bottom-to-top, ref[2n] corner,
-// ref[2n+1..4n] top then top-right.  (x0, y0) are the block's coordinates
-// in the working area a (row stride as).
-__device__ __forceinline__ int32_t refValue(int i, int n, bool avAbove, bool avLeft, bool avAR, const uint8_t* a,
-                                            int as, int x0, int y0) {
-  // Each entry is one sample of the area: the left column L(r) = (x0-1, y0+r)
-  // (rows past n-1 repeat row n-1), the top row Tp(j) = (x0+j, y0-1) (past
-  // n-1 without above-right: Tp(n-1)), the corner; a missing side is
-  // replaced by the other side's nearest sample, both missing by kDCPred.
-  const int corner = 2 * n;
-  int ax, ay;
-  if (i < corner) {
-    ax = avLeft ? x0 - 1 : x0;
-    ay = avLeft ? y0 + min(corner - 1 - i, n - 1) : y0 - 1;
-  } else if (i == corner) {
-    ax = avLeft ? x0 - 1 : x0;
-    ay = avAbove ? y0 - 1 : y0;
-  } else {
-    const int j = i - corner - 1;
-    ax = avAbove ? x0 + ((j < n || avAR) ? j : n - 1) : x0 - 1;
-    ay = avAbove ? y0 - 1 : y0;
+// The neighbours of one n x n block as predictIntra sees them after
+// substituteRefs (ebiv/predict.go:131-219): top[j] is the sample above column
+// j, top[-1] the corner, col[r] the one left of row r.  A missing side is
+// replaced by the other side's nearest sample, both missing by kDCPred; past
+// n - 1 the left column repeats, and the top row does without above-right.
+template <int N>
+struct IntraRefs {
+  const uint8_t* top;
+  const uint8_t* col;
+  bool above, left, aboveRight;
+  __device__ __forceinline__ int t(int j) const {
+    return above ? top[(j < N || aboveRight) ? j : N - 1] : (left ? col[0] : kDCPred);
   }
-  return (avLeft || avAbove) ? (int32_t)a[ay * as + ax] : kDCPred;
+  __device__ __forceinline__ int l(int r) const { return left ? col[min(r, N - 1)] : (above ? top[0] : kDCPred); }
+  __device__ __forceinline__ int corner() const {
+    return left ? (above ? top[-1] : col[0]) : (above ? top[0] : kDCPred);
+  }
+  // Samples j to j + 3 (j a multiple of 4, below N).
+  __device__ __forceinline__ uint32_t top4(int j) const {
+    return above ? *reinterpret_cast<const uint32_t*>(top + j) : 0x01010101u * (uint32_t)(left ? col[0] : kDCPred);
+  }
+  __device__ __forceinline__ uint32_t left4(int r) const {
+    return left ? *reinterpret_cast<const uint32_t*>(col + r) : 0x01010101u * (uint32_t)(above ? top[0] : kDCPred);
+  }
+};
+
+// Predicts and reconstructs P samples of an N x N block, row r from column c
+// on (predictIntra, ebiv/predict.go:131-219), into the bytes of the result;
+// res is null or their residual.
+template <int N, int P>
+__device__ __forceinline__ uint32_t intraSamples(const IntraRefs<N>& f, int mode, int r, int c, const int32_t* res) {
+  int v[P];
+  int32_t add[P];
+#pragma unroll
+  for (int i = 0; i < P; i++) add[i] = 0;
+  if (res) {
+    if (P == 4) {
+      const int4 q = *reinterpret_cast<const int4*>(res);
+      add[0] = q.x;
+      add[P / 4] = q.y;
+      add[P / 2] = q.z;
+      add[3 * P / 4] = q.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < P; i++) add[i] = res[i];
+    }
+  }
+  if (mode == modeDC) {
+    uint32_t sum = N;
+#pragma unroll
+    for (int i = 0; i < N; i += 4) sum = __dp4a(f.left4(i), 0x01010101u, __dp4a(f.top4(i), 0x01010101u, sum));
+#pragma unroll
+    for (int i = 0; i < P; i++) v[i] = (int)(sum / (2 * N));
+  } else if (mode == modeV || mode == modeTM) {
+    const int d = mode == modeTM ? f.l(r) - f.corner() : 0;
+    const uint32_t t = P == 4 ? f.top4(c) : 0u;
+#pragma unroll
+    for (int i = 0; i < P; i++) v[i] = clampByteD((P == 4 ? (int)((t >> (8 * i)) & 0xFF) : f.t(c + i)) + d);
+  } else if (mode == modeH) {
+    v[0] = f.l(r);
+#pragma unroll
+    for (int i = 1; i < P; i++) v[i] = v[0];
+  } else {
+    // An angle: position (a + 1) * angle / 32 along the main side (the top
+    // row of a vertical mode), continued on the other side below 0.
+    const bool vertical = mode == modeD45 || mode == modeD27 || mode == modeD23;
+    const int angle = mode == modeD45 || mode == modeD135 ? 32 : (mode == modeD27 || mode == modeD117 ? 13 : -13);
+    constexpr int kInv = -630;  // of -13
+    auto ext = [&](int k) __attribute__((always_inline)) {
+      if (k == 0) return f.corner();
+      if (k > 2 * N) return 0;
+      if (k > 0) return vertical ? f.t(k - 1) : f.l(k - 1);
+      const int t = (k * kInv + 128) >> 8;
+      return t == 0 ? f.corner() : (vertical ? f.l(t - 1) : f.t(t - 1));
+    };
+    uint32_t o = 0;
+#pragma unroll 1  // for the size of the code (see kIntraRecon)
+    for (int i = 0; i < P; i++) {
+      const int pos = ((vertical ? r : c + i) + 1) * angle, idx = pos >> 5, fact = pos & 31;
+      const int k = (vertical ? c + i : r) + idx;
+      const int a = ((32 - fact) * ext(k + 1) + fact * ext(k + 2) + 16) >> 5;
+      o |= (uint32_t)clampByteD(wadd(a, res ? res[i] : 0)) << (8 * i);
+    }
+    return o;
+  }
+  uint32_t o = 0;
+#pragma unroll
+  for (int i = 0; i < P; i++) o |= (uint32_t)clampByteD(wadd(v[i], add[i])) << (8 * i);
+  return o;
 }
 
-// Predicts and reconstructs one n x n block (predictIntra,
-// ebiv/predict.go:131-219) at area coordinates (ax, ay) of working area a,
-// writing each sample to the area and to plane p at (px, py).  Lanes l of nl
-// (a half warp or the whole warp) share the block; every lane of the warp
-// calls it, with active false where its half has no block this step, so
-// both __syncwarp barriers see the full warp.
-__device__ void intraBlock(int32_t* ref, uint8_t* a, int as, int ax, int ay, uint8_t* p, int stride, int px, int py,
-                           int n, int mode, bool avAbove, bool avLeft, bool avAR, const int32_t* res, int resStride,
-                           int l, int nl, bool active) {
-  const int corner = 2 * n;
-  if (active)
-    for (int i = l; i <= 4 * n; i += nl) ref[i] = refValue(i, n, avAbove, avLeft, avAR, a, as, ax, ay);
-  __syncwarp();
-  if (!active) {
-    __syncwarp();
-    return;
-  }
-  // n is 4, 8 or 16: shifts instead of divisions, and the DC sum's loads
-  // issued together (unrolled, predicated past n).
-  const int lg = n == 4 ? 2 : (n == 8 ? 3 : 4);
-  int32_t dc = 0;
-  if (mode == modeDC) {
-    int32_t sum = 0;
+// Four samples of a plane: one word when the plane's words are aligned (always
+// but for the planes that a caller of ebivgpu_decode_key_noalloc may give).
+__device__ __forceinline__ void storeQuad(uint8_t* p, uint32_t o, bool words) {
+  if (words) {
+    *reinterpret_cast<uint32_t*>(p) = o;
+  } else {
 #pragma unroll
-    for (int i = 0; i < 16; i++)
-      if (i < n) sum += ref[corner + 1 + i] + ref[corner - 1 - i];
-    dc = (sum + n) >> (lg + 1);  // sum >= 0: the division by 2n
+    for (int i = 0; i < 4; i++) p[i] = (uint8_t)(o >> (8 * i));
   }
-  int angle = 0, inv = 0;
-  bool vertical = false;
-  switch (mode) {
-    case modeD45: angle = 32; vertical = true; break;
-    case modeD27: angle = 13; vertical = true; break;
-    case modeD23: angle = -13; inv = -630; vertical = true; break;
-    case modeD135: angle = 32; break;
-    case modeD117: angle = 13; break;
-    case modeD113: angle = -13; inv = -630; break;
-    default: break;
-  }
-  const int nn = n * n;
-  for (int o = l; o < nn; o += nl) {
-    const int r = o >> lg, c = o & (n - 1);
-    int32_t v;
-    switch (mode) {
-      case modeV: v = ref[corner + 1 + c]; break;
-      case modeH: v = ref[corner - 1 - r]; break;
-      case modeTM: v = clampByteD(ref[corner + 1 + c] + ref[corner - 1 - r] - ref[corner]); break;
-      case modeDC: v = dc; break;
-      default: {
-        const int aa = vertical ? r : c, b = vertical ? c : r;
-        const int pos = (aa + 1) * angle;
-        const int idx = pos >> 5, fact = pos & 31;
-        auto ext = [&](int k) -> int32_t {
-          if (k >= 0) {
-            if (k > 2 * n) return 0;
-            return vertical ? ref[corner + k] : ref[corner - k];
-          }
-          const int t = (k * inv + 128) >> 8;
-          return vertical ? ref[corner - t] : ref[corner + t];
-        };
-        v = ((32 - fact) * ext(b + idx + 1) + fact * ext(b + idx + 2) + 16) >> 5;
+}
+__device__ __forceinline__ uint32_t loadQuad(const uint8_t* p, bool words) {
+  if (words) return *reinterpret_cast<const uint32_t*>(p);
+  return (uint32_t)p[0] | (uint32_t)p[1] << 8 | (uint32_t)p[2] << 16 | (uint32_t)p[3] << 24;
+}
+
+// One N x N luma block at (x, y) of its macroblock, by lanes l of nl: into the
+// plane at p (the block's first sample) and where later blocks look for it.
+template <int N>
+__device__ __forceinline__ void intraLumaBlock(IntraScratch& S, int x, int y, int mode, bool above, bool left,
+                                               bool aboveRight, bool hasRes, uint8_t* p, int stride, bool words, int l,
+                                               int nl) {
+  const IntraRefs<N> f = {S.areaY + y * kAreaW + kAreaX + x, S.colY[x >> 2] + y, above, left, aboveRight};
+  // As many lanes as there are: a 4x4 block has a sample for each of its half
+  // warp's, an 8x8 one two for each of the warp's, a 16x16 one words.
+  constexpr int P = N == 4 ? 1 : (N == 8 ? 2 : 4);
+#pragma unroll 1
+  for (int q = l; q < N * N / P; q += nl) {
+    const int r = q / (N / P), c = P * (q % (N / P));
+    const uint32_t o = intraSamples<N, P>(f, mode, r, c, hasRes ? S.res + (y + r) * 16 + x + c : nullptr);
+    uint8_t* const to = p + (size_t)r * stride + c;
+    if (P == 4) {
+      storeQuad(to, o, words);
+    } else {
+#pragma unroll
+      for (int i = 0; i < P; i++) {
+        const uint8_t v = (uint8_t)(o >> (8 * i));
+        to[i] = v;
+        if ((r & 3) == 3) S.areaY[(1 + y + r) * kAreaW + kAreaX + x + c + i] = v;
+        if (((c + i) & 3) == 3) S.colY[(x + c + i + 1) >> 2][y + r] = v;
       }
     }
-    v = res ? clampByteD(wadd(v, res[r * resStride + c])) : clampByteD(v);
-    a[(ay + r) * as + ax + c] = (uint8_t)v;  // the block's reference array is already in ref
-    p[(size_t)(py + r) * stride + px + c] = (uint8_t)v;
   }
-  __syncwarp();
 }
 
 // Progress of the intra macroblocks of one tile, shared by the warps of its
@@ -1607,16 +1653,15 @@ struct IntraSync {
         *abort = 1;
         break;
       }
-      __nanosleep(64);
+      __nanosleep(20);
     }
     __threadfence_block();
   }
   // Publishes progress v once every lane's writes so far are visible to the CTA.
   __device__ __forceinline__ void publish(volatile uint8_t* p, int v, int lane) const {
-    __threadfence_block();
     __syncwarp();
     if (lane == 0) {
-      __threadfence_block();
+      __threadfence_block();  // and with it the other lanes' writes, which the barrier ordered before
       *p = (uint8_t)v;
     }
   }
@@ -1629,7 +1674,7 @@ struct IntraSync {
 // macroblocks done and the above-right one past step 6 (its block (0,3),
 // the only one the top-right block reads).  Other transform sizes wait for
 // all four neighbours to be done.
-__device__ void intraLuma(const ReconView& f, IntraScratch& S, const IntraSync& sy, int mbx, int mby, int lane) {
+__device__ __forceinline__ void intraLuma(const ReconView& f, IntraScratch& S, const IntraSync& sy, int mbx, int mby, int lane) {
   const int idx = mby * f.mbCols + mbx;
   RecRegs r;
   r.load(f.mbrec + idx);
@@ -1637,7 +1682,7 @@ __device__ void intraLuma(const ReconView& f, IntraScratch& S, const IntraSync& 
   const uint32_t wm = r.wmask();
   if (!wm) return;
   const uint32_t nzm = r.nzmask();
-  const int tx = r.tx(), n = 4 << tx, per = 4 >> tx, nb = per * per;
+  const int tx = r.tx(), per = 4 >> tx, nb = per * per;
   const int tileLeft = sy.x0 * 16, tileTop = sy.y0 * 16, tileRight = sy.x1 * 16;
   const int mbLeft = mbx * 16, mbTop = mby * 16, mbRight = mbLeft + 16;
   uint8_t* const Y = f.rec[0];
@@ -1682,38 +1727,43 @@ __device__ void intraLuma(const ReconView& f, IntraScratch& S, const IntraSync& 
   bool leftNow = false;
   if (left) leftNow = __shfl_sync(kFull, *leftP >= kLumaDone ? 1 : 0, 0) != 0;
   if (leftNow) __threadfence_block();
-  const int xa = mbLeft - 1 + lane;
-  const bool haveA = up && xa >= tileLeft && xa < tileRight;
-  const bool haveB = up && lane == 0 && mbLeft + 31 < tileRight;  // area entry 32
-  const uint8_t* const rowAbove = Y + (size_t)(mbTop - 1) * ys;
-  uint8_t a0 = 0, a1 = 0, lc = 0;
-  if (haveA) a0 = rowAbove[xa];
-  if (haveB) a1 = rowAbove[mbLeft + 31];
+  // The row above in words: lane 0 the four samples left of the macroblock,
+  // lanes 1-4 above it, lanes 5-8 right of it.
+  const bool haveA = up && (lane == 0 ? left : lane <= 4 || (lane <= 8 && mbRight < tileRight));
+  uint32_t a0 = 0;
+  uint8_t lc = 0;
+  if (haveA) a0 = loadQuad(Y + (size_t)(mbTop - 1) * ys + mbLeft - 4 + 4 * lane, f.words);
   if (leftNow && lane < 16) lc = Y[(size_t)(mbTop + lane) * ys + mbLeft - 1];
   if (lumaRes)
 #pragma unroll
     for (int q = 0; q < 8; q++) S.res[lane + 32 * q] = rv[q];
-  if (haveA) S.areaY[lane] = a0;
-  if (haveB) S.areaY[32] = a1;
-  if (leftNow && lane < 16) S.areaY[(1 + lane) * kAreaW] = lc;
-  auto block = [&](int k, int l, int nl, bool active, int half) {
-    const int bx = (k & (per - 1)) << (2 + tx), by = (k >> (2 - tx)) << (2 + tx);  // per = 4 >> tx, n = 4 << tx
+  if (haveA) *reinterpret_cast<uint32_t*>(S.areaY + kAreaX - 4 + 4 * lane) = a0;
+  if (leftNow && lane < 16) S.colY[0][lane] = lc;
+  // The corner of blocks below the first row, at the macroblock's left edge:
+  // the sample left of and above them, in the area's column left of x = 0.
+  if (leftNow && lane < 16 && (lane & 3) == 3) S.areaY[(1 + lane) * kAreaW + kAreaX - 1] = lc;
+  auto block = [&](auto size, int k, int l, int nl) __attribute__((always_inline)) {
+    constexpr int n = decltype(size)::value;
+    constexpr int kPer = 16 / n;
+    const int bx = k % kPer * n, by = k / kPer * n;
     const int x0 = mbLeft + bx, y0 = mbTop + by;
-    const bool avAbove = y0 > tileTop, avLeft = x0 > tileLeft;
-    bool avAR = false;
-    if (!(y0 <= tileTop || x0 + 2 * n > tileRight)) avAR = (y0 == mbTop) ? true : (x0 + 2 * n <= mbRight);
-    const bool hasRes = (nzm >> k) & 1;
-    intraBlock(S.ref[half], S.areaY, kAreaW, 1 + bx, 1 + by, Y, ys, x0, y0, n, active ? r.lmode(k) : 0, avAbove,
-               avLeft, avAR, hasRes ? S.res + by * 16 + bx : nullptr, 16, l, nl, active);
+    const bool avAR = y0 > tileTop && x0 + 2 * n <= tileRight && (by == 0 || x0 + 2 * n <= mbRight);
+    intraLumaBlock<n>(S, bx, by, r.lmode(k), y0 > tileTop, x0 > tileLeft, avAR, (nzm >> k) & 1,
+                      Y + (size_t)y0 * ys + x0, ys, f.words, l, nl);
   };
   if (tx == 0) {
     // Blocks beyond the first unwritten one (a prefix in raster order) are
     // skipped; each step is published all the same.
     const int half = lane >> 4;
+#pragma unroll 1
     for (int t = 0; t < 10; t++) {
       if (left && !leftNow && !(t & 1) && t <= 6) {  // left column rows 2t..2t+3, for block (0, t/2)
         sy.wait(leftP, t + 4);
-        if (lane < 4) S.areaY[(1 + 2 * t + lane) * kAreaW] = Y[(size_t)(mbTop + 2 * t + lane) * ys + mbLeft - 1];
+        if (lane < 4) {
+          const uint8_t v = Y[(size_t)(mbTop + 2 * t + lane) * ys + mbLeft - 1];
+          S.colY[0][2 * t + lane] = v;
+          if (lane == 3) S.areaY[(4 + 2 * t) * kAreaW + kAreaX - 1] = v;
+        }
       }
       __syncwarp();
       int k = -1, seen = 0;
@@ -1724,22 +1774,24 @@ __device__ void intraLuma(const ReconView& f, IntraScratch& S, const IntraSync& 
           seen++;
         }
       }
-      const bool active = k >= 0 && ((wm >> k) & 1);
-      block(active ? k : 0, lane & 15, 16, active, half);
+      if (k >= 0 && ((wm >> k) & 1)) block(std::integral_constant<int, 4>(), k, lane & 15, 16);
       sy.publish(own, t + 1, lane);
     }
   } else {
     __syncwarp();  // the left column was loaded with the row above
+#pragma unroll 1
     for (int k = 0; k < nb; k++) {
       if (!((wm >> k) & 1)) break;
-      block(k, lane, 32, true, 0);
+      if (tx == 1) block(std::integral_constant<int, 8>(), k, lane, 32);
+      else block(std::integral_constant<int, 16>(), k, lane, 32);
+      __syncwarp();
     }
   }
 }
 
 // The chroma of an intra macroblock: waits for the left, above-left and
 // above macroblocks' chroma (chroma prediction reads no above-right samples).
-__device__ void intraChroma(const ReconView& f, IntraScratch& S, const IntraSync& sy, int mbx, int mby, int lane) {
+__device__ __forceinline__ void intraChroma(const ReconView& f, IntraScratch& S, const IntraSync& sy, int mbx, int mby, int lane) {
   const int idx = mby * f.mbCols + mbx;
   RecRegs r;
   r.load(f.mbrec + idx);
@@ -1771,37 +1823,28 @@ __device__ void intraChroma(const ReconView& f, IntraScratch& S, const IntraSync
     sy.wait(sy.chroma + sy.at(mbx, mby - 1), 1);
   }
   if (left) sy.wait(sy.chroma + sy.at(mbx - 1, mby), 1);
-  const int cl = mbx * 8, ct = mby * 8;
-  // Both planes' row above and left column, loaded together.
-  const bool haveT = up && lane < 9 && (lane > 0 || left), haveL = left && lane < 8;
-  uint8_t t0 = 0, t1 = 0, l0 = 0, l1 = 0;
-  if (haveT) {
-    t0 = f.rec[1][(size_t)(ct - 1) * cs + cl - 1 + lane];
-    t1 = f.rec[2][(size_t)(ct - 1) * cs + cl - 1 + lane];
-  }
-  if (haveL) {
-    l0 = f.rec[1][(size_t)(ct + lane) * cs + cl - 1];
-    l1 = f.rec[2][(size_t)(ct + lane) * cs + cl - 1];
-  }
+  // A half warp per plane: the row above with its corner (words left of and
+  // above the block) and the left column, then the block's sixteen words.
+  const int pl = lane >> 4, l = lane & 15;
+  uint8_t* const P = (pl ? f.rec[2] : f.rec[1]) + (size_t)(mby * 8) * cs + mbx * 8;
+  const bool haveT = up && l < 3 && (l > 0 || left), haveL = left && l >= 8;
+  uint32_t t = 0;
+  uint8_t lc = 0;
+  if (haveT) t = loadQuad(P - cs + 4 * l - 4, f.words);
+  if (haveL) lc = P[(size_t)(l - 8) * cs - 1];
   if (chromaRes)
 #pragma unroll
     for (int q = 0; q < 4; q++) S.res[256 + lane + 32 * q] = rv[q];
-  if (haveT) {
-    S.areaC[0][lane] = t0;
-    S.areaC[1][lane] = t1;
-  }
-  if (haveL) {
-    S.areaC[0][(1 + lane) * 16] = l0;
-    S.areaC[1][(1 + lane) * 16] = l1;
-  }
+  if (haveT) *reinterpret_cast<uint32_t*>(S.topC[pl] + kAreaX - 4 + 4 * l) = t;
+  if (haveL) S.colC[pl][l - 8] = lc;
   __syncwarp();
-  const int cmode = r.cmode();
-  for (int pl = 0; pl < 2; pl++) {
-    const uint32_t bit = 1u << (16 + pl);
-    if (!(wm & bit)) break;
-    const bool hasRes = (nzm & bit) != 0;
-    intraBlock(S.ref[0], S.areaC[pl], 16, 1, 1, f.rec[1 + pl], cs, mbx * 8, mby * 8, 8, cmode, up, left, false,
-               hasRes ? S.res + 256 + pl * 64 : nullptr, 8, lane, 32, true);
+  // Cr is written only after Cb.
+  if (pl == 0 ? (wm >> 16) & 1 : (wm >> 16) == 3) {
+    const IntraRefs<8> refs = {S.topC[pl] + kAreaX, S.colC[pl], up, left, false};
+    const int row = l >> 1, c = 4 * (l & 1);
+    storeQuad(P + (size_t)row * cs + c,
+              intraSamples<8, 4>(refs, r.cmode(), row, c, (nzm >> (16 + pl)) & 1 ? S.res + 256 + pl * 64 + row * 8 + c : nullptr),
+              f.words);
   }
 }
 
@@ -1818,16 +1861,30 @@ constexpr int kIntraSortBytes = 64 * 1024;
 // for and interleaves the rows the way the dependencies allow.
 __device__ __forceinline__ int intraKey(int x, int y) { return 4 * x + 11 * y; }
 
-// One CTA of W warps per tile, a dataflow schedule: the warps take the
-// tile's intra macroblocks' luma and chroma as jobs in wavefront order
-// (intraKey; raster order when the tile's ordering does not fit sortInts)
-// and each job waits for exactly the neighbouring samples it predicts from
-// (IntraSync).  Either order lists every job after the jobs it waits for, so
-// the earliest unfinished job can always proceed.  The residuals were
-// computed by kInterRecon phase 0.  Dynamic shared memory: W IntraScratch,
-// 2 * flagMBs progress bytes (rounded to 16), sortInts words for the
-// ordering.  Few tiles take 16 warps per CTA; many tiles fewer, so that
-// several CTAs share an SM.
+// One CTA of W warps per tile, or two (gridDim.y), one for luma and one for
+// both chroma planes, neither of which reads the other's samples: a dataflow
+// schedule.  The warps take the tile's intra macroblocks' luma and chroma as
+// jobs in wavefront order (intraKey; raster order when the tile's ordering
+// does not fit sortInts) and each job waits for exactly the neighbouring
+// samples it predicts from (IntraSync).  Either order lists every job after
+// the jobs it waits for, so the earliest unfinished job can always proceed.
+// The residuals were computed by kInterRecon phase 0.  Dynamic shared memory:
+// W IntraScratch, 2 * flagMBs progress bytes (rounded to 16), sortInts words
+// for the ordering.
+//
+// A tile is bound by its warps' work, 550 instructions a job at 11 cycles
+// each, more than by the chain of its dependencies (a 40x23 key tile takes 1.6
+// times as long with 8 warps as with 16), so few tiles take two CTAs of 16
+// warps each; with more tiles than half the SMs, where two CTAs would have 8
+// warps each and luma more than half the work, one; with more than the SMs,
+// CTAs of fewer warps, several to an SM.  One CTA, and a reference array built
+// for every block: 390 us for four such tiles, 294 us for twelve of 30x22,
+// 2.54 ms for one of 80x45; two CTAs and the references read in place: 265,
+// 225 us and 1.57 ms.  One CTA a tile, 120 tiles of 40x23: 401 us, now 356.
+//
+// The code is kept small: with the samples of an angle unrolled it leaves the
+// SMs' instruction caches, and many SMs fetch it from the L2 (690 us for the
+// 120 tiles, 280 us for four).
 template <int W>
 __global__ void __launch_bounds__(32 * W, 16 / W)
     kIntraRecon(const FrameDesc* frames, const int2* jobs, int njobs, int flagMBs, int sortInts) {
@@ -1851,6 +1908,9 @@ __global__ void __launch_bounds__(32 * W, 16 / W)
   const TileRange tr = f.tiles[tile];
   const int tw = tr.mbX1 - tr.mbX0, th = tr.mbY1 - tr.mbY0, tmbs = tw * th;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+  // The planes of this CTA: each has its own progress, also where two CTAs
+  // keep it in the same global memory.
+  const bool both = gridDim.y == 1, lumaHere = both || blockIdx.y == 0, chromaHere = both || blockIdx.y == 1;
   uint8_t* flags;
   if (tmbs <= flagMBs) {
     flags = sDyn + sizeof(IntraScratch) * W;
@@ -1870,8 +1930,8 @@ __global__ void __launch_bounds__(32 * W, 16 / W)
   sy.tw = tw;
   const uint32_t* list = f.intraList + tr.mbBase;
   for (int i = tid; i < tmbs; i += blockDim.x) {
-    sy.luma[i] = kLumaDone;
-    sy.chroma[i] = 1;
+    if (lumaHere) sy.luma[i] = kLumaDone;
+    if (chromaHere) sy.chroma[i] = 1;
   }
   if (tid == 0) {
     sNext = 0;
@@ -1882,8 +1942,8 @@ __global__ void __launch_bounds__(32 * W, 16 / W)
   for (int i = tid; i < n; i += blockDim.x) {
     const int idx = (int)(list[i] & kIndexMask);
     const int m = sy.at(idx % mbCols, idx / mbCols);
-    sy.luma[m] = 0;
-    sy.chroma[m] = 0;
+    if (lumaHere) sy.luma[m] = 0;
+    if (chromaHere) sy.chroma[m] = 0;
   }
   __syncthreads();
   // Wavefront order: a counting sort of the list by intraKey in shared memory.
@@ -1945,14 +2005,15 @@ __global__ void __launch_bounds__(32 * W, 16 / W)
   ReconView view;
   view.load(f);
   IntraScratch& S = sS[warp];
+  const int jobsHere = both ? 2 * n : n;
   for (;;) {
     int k = 0;
     if (lane == 0) k = atomicAdd(&sNext, 1);
     k = __shfl_sync(kFull, k, 0);
-    if (k >= 2 * n) break;
-    const int idx = (int)(order[k >> 1] & kIndexMask);
+    if (k >= jobsHere) break;
+    const int idx = (int)(order[both ? k >> 1 : k] & kIndexMask);
     const int mbx = idx % mbCols, mby = idx / mbCols;
-    if (k & 1) {
+    if (both ? k & 1 : (int)blockIdx.y) {
       intraChroma(view, S, sy, mbx, mby, lane);
       sy.publish(sy.chroma + sy.at(mbx, mby), 1, lane);
     } else {
@@ -2043,11 +2104,11 @@ static void allowIntraSmem() {
 }
 
 template <int W>
-static void launchIntraW(const FrameDesc* frames, const int2* jobs, int njobs, int flagMBs, int sortInts,
+static void launchIntraW(const FrameDesc* frames, const int2* jobs, int njobs, int ctas, int flagMBs, int sortInts,
                          cudaStream_t s) {
   constexpr size_t kScratch = sizeof(dev::IntraScratch) * W;
   const size_t smem = kScratch + (((size_t)2 * flagMBs + 15) & ~(size_t)15) + 4 * (size_t)sortInts;
-  launchDependent(dev::kIntraRecon<W>, dim3(njobs), dim3(32 * W), smem, s, frames, jobs, njobs, flagMBs, sortInts);
+  launchDependent(dev::kIntraRecon<W>, dim3(njobs, ctas), dim3(32 * W), smem, s, frames, jobs, njobs, flagMBs, sortInts);
 }
 
 // maxTileMBs: the largest tile of the launch's frames, in macroblocks;
@@ -2079,13 +2140,14 @@ void launchIntra(const FrameDesc* frames, const int2* jobs, int njobs, int maxTi
   const int flagMBs = std::max(1, std::min(maxTileMBs, dev::kIntraFlagMBs));
   int sortInts = std::max(0, maxTileMBs) + std::max(0, maxTileKeys);
   if (4 * (size_t)sortInts > (size_t)dev::kIntraSortBytes) sortInts = 0;  // raster order
+  const int ctas = 2 * njobs <= nsm ? 2 : 1;  // per tile
   if (warps != 4 && warps != 8 && warps != 16) warps = njobs <= nsm ? 16 : (njobs <= 2 * nsm ? 8 : 4);
   if (warps == 16)
-    launchIntraW<16>(frames, jobs, njobs, flagMBs, sortInts, s);
+    launchIntraW<16>(frames, jobs, njobs, ctas, flagMBs, sortInts, s);
   else if (warps == 8)
-    launchIntraW<8>(frames, jobs, njobs, flagMBs, sortInts, s);
+    launchIntraW<8>(frames, jobs, njobs, ctas, flagMBs, sortInts, s);
   else
-    launchIntraW<4>(frames, jobs, njobs, flagMBs, sortInts, s);
+    launchIntraW<4>(frames, jobs, njobs, ctas, flagMBs, sortInts, s);
 }
 
 }  // namespace ebiv

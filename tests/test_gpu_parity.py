@@ -192,3 +192,13 @@ def test_vector_prediction_by_tile_shape(gpu_required, w, h):
     at once: 1, 2, 3, 7, 9, 128 and 129 macroblocks wide, up to 32 rows and more."""
     cont, _, rec = encode_gen(w, h, 3, ebiv.synth_pan, intra=20, gop=3, tiles=(1, 1))
     _check(cont, w, h, rec)
+
+
+@pytest.mark.parametrize("grid", [(4, 4), (19, 4), (11, 7), (19, 8), (17, 9), (19, 16), (20, 16)])
+@pytest.mark.parametrize("qp", [10, 34])
+def test_intra_stage_by_tile_count(gpu_required, grid, qp):
+    """Key frames and an inter frame of as many tiles as lie on both sides of each of the intra stage's launch
+    shapes on 152 SMs: two CTAs a tile up to 76 tiles, then one of 16, 8 (above 152) or 4 warps (above 304)."""
+    w, h = 32 * grid[0] + 21, 32 * grid[1] + 9
+    cont, _, rec = encode_gen(w, h, 2, ebiv.synth_frame, intra=qp, gop=2, tiles=grid)
+    _check(cont, w, h, rec)

@@ -143,3 +143,30 @@ def test_size_limits_and_frame_types_are_refused_before_device_work():
     assert _dims(inter)[0] == EBIV_ERR_NOKEYFRAME
     assert _dims(b"")[0] == EBIV_ERR_CORRUPT
     assert b"no-allocation" in _native.lib().ebivgpu_status_string(EBIV_ERR_TOO_LARGE)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shift,wider", [(0, 1), (1, 0), (3, 3), (2, 5), (4, 4)])
+def test_planes_of_any_alignment(gpu_required, shift, wider):
+    """Planes that start at and have strides of any number of bytes: reconstruction stores words only where they
+    are aligned."""
+    import torch
+
+    for pkt in (_packets("odd_37x21")[0], _packets("scene_160x96")[0]):
+        want = ebiv_oracle.decode_all([pkt])[0][1]
+        st, w, h = _dims(pkt)
+        assert st == 0
+        cols, rows = (w + 15) // 16, (h + 15) // 16
+        ys, cs = cols * 16 + wider, cols * 8 + wider
+        buf = torch.full((3, rows * 16 * ys + 8), 0xAB, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        ow, oh = C.c_int32(), C.c_int32()
+        at = [buf[k].data_ptr() + shift for k in range(3)]
+        assert _native.lib().ebivgpu_decode_key_noalloc(pkt, len(pkt), at[0], ys, rows * 16 * ys, at[1], at[2], cs,
+                                                        rows * 8 * cs, None, C.byref(ow), C.byref(oh)) == 0
+        cw, ch = (w + 1) // 2, (h + 1) // 2
+        host = buf.cpu().numpy()
+        got = b"".join(np.ascontiguousarray(host[k, shift:shift + r * s].reshape(r, s)[:vh, :vw]).tobytes()
+                       for k, r, s, vw, vh in ((0, rows * 16, ys, w, h), (1, rows * 8, cs, cw, ch), (2, rows * 8, cs, cw, ch)))
+        assert got == want
+        assert (host[0, :shift] == 0xAB).all() and (host[0, shift + rows * 16 * ys:] == 0xAB).all()
