@@ -71,32 +71,24 @@ template <>
 __device__ __forceinline__ float fromF<float>(float v) { return v; }
 
 // ---------------------------------------------------------------------------
-// 3x3 convolution, zero padding 1, one thread per two output pixels (one
-// below the other) and all CO output channels in registers.  in [B][CI][h][w],
-// w [CO][CI][9] (BF16), out [B][CO][h][w].  bias may be null; relu clamps at
-// zero; mask (same shape as out, BF16) zeroes outputs where mask <= 0 (the
-// ReLU derivative of the layer below, for the data gradient).  An output sums
-// its products in FP32 over channels, then taps, in that order.
-//
-// Bound by the FP32 multiply-adds: the weights lie in shared memory with the
-// output channels side by side, so that one 16-byte load feeds eight of them.
-// 480x272, 32 to 32 channels: 190 us with a load of its own for every product
-// and one pixel a thread, 111 us now.
+// 3x3 convolution, zero padding 1, one thread per output pixel and all CO
+// output channels in registers.  in [B][CI][h][w], w [CO][CI][9] (BF16),
+// out [B][CO][h][w].  bias may be null; relu clamps at zero; mask (same
+// shape as out, BF16) zeroes outputs where mask <= 0 (the ReLU derivative
+// of the layer below, for the data gradient).
 // ---------------------------------------------------------------------------
-constexpr int kConvThreads = kTile * kTile / 2;
 template <int CO, class TIn, class TOut>
-__global__ void __launch_bounds__(kConvThreads) kConv3x3(const TIn* __restrict__ in, int CI, const bf16* __restrict__ wt,
+__global__ void __launch_bounds__(kTile* kTile) kConv3x3(const TIn* __restrict__ in, int CI, const bf16* __restrict__ wt,
                                                          const float* __restrict__ bias, TOut* __restrict__ out,
                                                          const bf16* __restrict__ mask, int relu, int h, int w) {
-  constexpr int kPad = (CO + 3) & ~3;
   __shared__ float sIn[kChunk][kTile + 2][kTile + 2];
-  __shared__ __align__(16) float sW[kChunk][9][kPad];
-  const int tx = threadIdx.x % kTile, ty = 2 * (threadIdx.x / kTile);
+  __shared__ float sW[CO][kChunk][9];
+  const int tx = threadIdx.x % kTile, ty = threadIdx.x / kTile;
   const int x0 = blockIdx.x * kTile, y0 = blockIdx.y * kTile, b = blockIdx.z;
-  const int x = x0 + tx;
-  float acc[2][CO];
+  const int x = x0 + tx, y = y0 + ty;
+  float acc[CO];
 #pragma unroll
-  for (int c = 0; c < CO; c++) acc[0][c] = acc[1][c] = 0.f;
+  for (int c = 0; c < CO; c++) acc[c] = 0.f;
   const TIn* inB = in + (size_t)b * CI * h * w;
   for (int c0 = 0; c0 < CI; c0 += kChunk) {
     const int nc = min(kChunk, CI - c0);
@@ -108,48 +100,28 @@ __global__ void __launch_bounds__(kConvThreads) kConv3x3(const TIn* __restrict__
       if (yy >= 0 && yy < h && xx >= 0 && xx < w) v = toF(inB[((size_t)(c0 + c) * h + yy) * w + xx]);
       sIn[c][rem / (kTile + 2)][rem % (kTile + 2)] = v;
     }
-    for (int i = threadIdx.x; i < nc * 9 * kPad; i += blockDim.x) {
-      const int co = i % kPad, rem = i / kPad;  // rem: channel * 9 + tap
-      sW[rem / 9][rem % 9][co] = co < CO ? __bfloat162float(wt[((size_t)co * CI + c0) * 9 + rem]) : 0.f;
+    for (int i = threadIdx.x; i < CO * nc * 9; i += blockDim.x) {
+      const int co = i / (nc * 9), rem = i % (nc * 9);
+      sW[co][rem / 9][rem % 9] = __bfloat162float(wt[((size_t)co * CI + c0 + rem / 9) * 9 + rem % 9]);
     }
     __syncthreads();
-#pragma unroll 1
-    for (int c = 0; c < nc; c++) {
-      float v[4][3];
-#pragma unroll
-      for (int r = 0; r < 4; r++)
-#pragma unroll
-        for (int q = 0; q < 3; q++) v[r][q] = sIn[c][ty + r][tx + q];
+    for (int c = 0; c < nc; c++)
 #pragma unroll
       for (int k = 0; k < 9; k++) {
-        const float a0 = v[k / 3][k % 3], a1 = v[k / 3 + 1][k % 3];
+        const float v = sIn[c][ty + k / 3][tx + k % 3];
 #pragma unroll
-        for (int co = 0; co < kPad; co += 4) {
-          const float4 q = *reinterpret_cast<const float4*>(&sW[c][k][co]);
-          const float f[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-          for (int u = 0; u < 4; u++)
-            if (co + u < CO) {
-              acc[0][co + u] = fmaf(a0, f[u], acc[0][co + u]);
-              acc[1][co + u] = fmaf(a1, f[u], acc[1][co + u]);
-            }
-        }
+        for (int co = 0; co < CO; co++) acc[co] = fmaf(v, sW[co][c][k], acc[co]);
       }
-    }
   }
+  if (x >= w || y >= h) return;
+  TOut* o = out + (size_t)b * CO * h * w + (size_t)y * w + x;
+  const bf16* m = mask ? mask + (size_t)b * CO * h * w + (size_t)y * w + x : nullptr;
 #pragma unroll
-  for (int p = 0; p < 2; p++) {
-    const int y = y0 + ty + p;
-    if (x >= w || y >= h) continue;
-    TOut* o = out + (size_t)b * CO * h * w + (size_t)y * w + x;
-    const bf16* m = mask ? mask + (size_t)b * CO * h * w + (size_t)y * w + x : nullptr;
-#pragma unroll
-    for (int co = 0; co < CO; co++) {
-      float v = acc[p][co] + (bias ? bias[co] : 0.f);
-      if (relu) v = fmaxf(v, 0.f);
-      if (m && !(__bfloat162float(m[(size_t)co * h * w]) > 0.f)) v = 0.f;
-      o[(size_t)co * h * w] = fromF<TOut>(v);
-    }
+  for (int co = 0; co < CO; co++) {
+    float v = acc[co] + (bias ? bias[co] : 0.f);
+    if (relu) v = fmaxf(v, 0.f);
+    if (m && !(__bfloat162float(m[(size_t)co * h * w]) > 0.f)) v = 0.f;
+    o[(size_t)co * h * w] = fromF<TOut>(v);
   }
 }
 
@@ -360,70 +332,37 @@ __global__ void kGather(const bf16* __restrict__ data, const int* __restrict__ i
 // [-R, R]^2 (full pels) with the smallest SAD between the current block and
 // the reference (coordinates clamped to the plane, as motion compensation
 // samples them).  Ties go to the zero vector, then to raster order, as the
-// encoder's exhaustive search scans.  One CTA per macroblock; a thread takes
-// four neighbouring vectors of a row at once, whose sixteen samples per line
-// it cuts from five aligned words, four samples to an instruction.  Bound by
-// those instructions: 1920x1088, R = 16, 728 us a search with a byte load per
-// sample, 96 us now.
+// encoder's exhaustive search scans.  One CTA per macroblock.
 // ---------------------------------------------------------------------------
 constexpr int kMaxR = 16;
-constexpr int kSearchThreads = 160;                  // R = 16: 33 rows of 9 groups in two rounds
-constexpr int kRefWords = (16 + 2 * kMaxR) / 4 + 1;  // a row of the window, one word more for the last group
-__device__ __forceinline__ uint32_t sad4(uint32_t a, uint32_t b, uint32_t sum) {
-  uint32_t d;
-  asm("vabsdiff4.u32.u32.u32.add %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sum));
-  return d;
-}
-__global__ void __launch_bounds__(kSearchThreads) kExhaustive(const uint8_t* __restrict__ cur,
-                                                              const uint8_t* __restrict__ ref, int stride, int W, int H,
-                                                              int mbCols, int R, int16_t* __restrict__ mvOut,
-                                                              int32_t* __restrict__ sadOut) {
-  __shared__ uint4 sCur[16];
-  __shared__ uint32_t sRef[(16 + 2 * kMaxR) * kRefWords];
+__global__ void __launch_bounds__(256) kExhaustive(const uint8_t* __restrict__ cur, const uint8_t* __restrict__ ref,
+                                                   int stride, int W, int H, int mbCols, int R,
+                                                   int16_t* __restrict__ mvOut, int32_t* __restrict__ sadOut) {
+  __shared__ uint8_t sCur[16][16];
+  __shared__ uint8_t sRef[16 + 2 * kMaxR][16 + 2 * kMaxR];
   __shared__ unsigned long long sBest;
   const int mb = blockIdx.x, mbx = mb % mbCols, mby = mb / mbCols;
   const int x0 = mbx * 16, y0 = mby * 16, span = 16 + 2 * R;
-  for (int i = threadIdx.x; i < 256; i += blockDim.x)
-    reinterpret_cast<uint8_t*>(sCur)[i] = cur[(size_t)(y0 + i / 16) * stride + x0 + i % 16];
-  for (int i = threadIdx.x; i < span * 4 * kRefWords; i += blockDim.x) {
-    const int r = i / (4 * kRefWords), c = i % (4 * kRefWords);
-    const int yy = min(max(y0 - R + r, 0), H - 1), xx = min(max(x0 - R + c, 0), W - 1);
-    reinterpret_cast<uint8_t*>(sRef)[i] = ref[(size_t)yy * stride + xx];
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) sCur[i / 16][i % 16] = cur[(size_t)(y0 + i / 16) * stride + x0 + i % 16];
+  for (int i = threadIdx.x; i < span * span; i += blockDim.x) {
+    const int yy = min(max(y0 - R + i / span, 0), H - 1), xx = min(max(x0 - R + i % span, 0), W - 1);
+    sRef[i / span][i % span] = ref[(size_t)yy * stride + xx];
   }
   if (threadIdx.x == 0) sBest = ~0ull;
   __syncthreads();
-  const int side = 2 * R + 1, groups = (side + 3) / 4;
+  const int n = (2 * R + 1) * (2 * R + 1);
   unsigned long long best = ~0ull;
-  for (int i = threadIdx.x; i < side * groups; i += blockDim.x) {
-    const int row = i / groups, col = 4 * (i % groups);
-    const uint32_t* p = sRef + row * kRefWords + col / 4;
-    uint32_t s[4] = {0u, 0u, 0u, 0u};
-#pragma unroll 4
-    for (int r = 0; r < 16; r++, p += kRefWords) {
-      const uint4 c = sCur[r];
-      const uint32_t w[5] = {p[0], p[1], p[2], p[3], p[4]};
+  for (int c = threadIdx.x; c < n; c += blockDim.x) {
+    const int dy = c / (2 * R + 1) - R, dx = c % (2 * R + 1) - R;
+    int s = 0;
+    for (int r = 0; r < 16; r++)
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
-        s[k] = sad4(c.x, __funnelshift_r(w[0], w[1], 8 * k), s[k]);
-        s[k] = sad4(c.y, __funnelshift_r(w[1], w[2], 8 * k), s[k]);
-        s[k] = sad4(c.z, __funnelshift_r(w[2], w[3], 8 * k), s[k]);
-        s[k] = sad4(c.w, __funnelshift_r(w[3], w[4], 8 * k), s[k]);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      if (col + k >= side) break;
-      const int c = row * side + col + k;
-      const unsigned rank = (row == R && col + k == R) ? 0u : (unsigned)c + 1u;  // zero first, then raster order
-      const unsigned long long key = ((unsigned long long)s[k] << 32) | rank;
-      best = key < best ? key : best;
-    }
+      for (int q = 0; q < 16; q++) s += abs((int)sCur[r][q] - (int)sRef[r + dy + R][q + dx + R]);
+    const unsigned rank = (dx == 0 && dy == 0) ? 0u : (unsigned)c + 1u;  // zero first, then raster order
+    const unsigned long long key = ((unsigned long long)(unsigned)s << 32) | rank;
+    best = key < best ? key : best;
   }
-  for (int o = 16; o; o >>= 1) {
-    const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
-    best = other < best ? other : best;
-  }
-  if ((threadIdx.x & 31) == 0) atomicMin(&sBest, best);
+  atomicMin(&sBest, best);
   __syncthreads();
   if (threadIdx.x == 0) {
     const unsigned rank = (unsigned)(sBest & 0xffffffffu);
@@ -576,7 +515,7 @@ int MvNet::exhaustive(const uint8_t* cur, const uint8_t* ref, int stride, int ra
       cudaMemcpy2DAsync(planes_ + (size_t)W_ * H_, W_, ref, stride, W_, H_, cudaMemcpyHostToDevice, stream_) !=
           cudaSuccess)
     return kErrDevice;
-  kExhaustive<<<mbs_, kSearchThreads, 0, stream_>>>(planes_, planes_ + (size_t)W_ * H_, W_, W_, H_, W_ / 16, range, mvs_, sads_);
+  kExhaustive<<<mbs_, 256, 0, stream_>>>(planes_, planes_ + (size_t)W_ * H_, W_, W_, H_, W_ / 16, range, mvs_, sads_);
   if (cudaMemcpyAsync(mv, mvs_, sizeof(int16_t) * 2 * mbs_, cudaMemcpyDeviceToHost, stream_) != cudaSuccess)
     return kErrDevice;
   if (sad && cudaMemcpyAsync(sad, sads_, sizeof(int32_t) * mbs_, cudaMemcpyDeviceToHost, stream_) != cudaSuccess)
@@ -621,7 +560,7 @@ int MvNet::gather(const int* idx, int batch) {
 
 void MvNet::forward(int batch) {
   const dim3 g((w_ + kTile - 1) / kTile, (h_ + kTile - 1) / kTile, batch);
-  const int T = kConvThreads;
+  const int T = kTile * kTile;
   const bf16* W0 = pbf_ + layerOffset(0);
   kConv3x3<kHidden, bf16, bf16><<<g, T, 0, stream_>>>(x0_, kInCh, W0, params_ + layerOffset(0) + layerWeights(0),
                                                       act_[0], nullptr, 1, h_, w_);
@@ -638,7 +577,7 @@ void MvNet::forward(int batch) {
 void MvNet::backward(int batch) {
   const dim3 g((w_ + kTile - 1) / kTile, (h_ + kTile - 1) / kTile, batch);
   const dim3 gw(1, (h_ + kTile * kBand - 1) / (kTile * kBand), batch);
-  const int T = kConvThreads;
+  const int T = kTile * kTile;
   // head: weights, then data gradient onto act[L-1] masked by its ReLU
   const int L = kLayers - 1;
   kConvWgrad<kHeadCh><<<gw, 256, 0, stream_>>>(act_[L - 1], kHidden, gHead_, grads_ + layerOffset(L),
