@@ -138,3 +138,15 @@ def test_proposed_encode_decodes_bit_exact_and_beats_no_net(gpu_required, traine
         for i, p in enumerate(pk):
             assert c.decode(p).packed() == want[i][1], f"{name} frame {i}"
     assert sizes["proposed"] < sizes["zero"], sizes
+
+
+@pytest.mark.parametrize("rng", [0, 1, 2, 4, 5, 15, 16])
+def test_exhaustive_search_of_any_range(gpu_required, rng):
+    """Ranges whose rows of vectors are not whole groups of the kernel's, the smallest and the largest, on noise
+    (every vector differs) and on a flat plane (every vector ties)."""
+    r = np.random.default_rng(rng)
+    net = mvnet.MvNet(48, 32)
+    for cur, ref in ((r.integers(0, 256, (32, 48), np.uint8), r.integers(0, 256, (32, 48), np.uint8)),
+                     (np.full((32, 48), 255, np.uint8), np.zeros((32, 48), np.uint8))):
+        mv, sad = net.exhaustive(cur, ref, rng)
+        assert [(int(s), int(x), int(y)) for s, (x, y) in zip(sad, mv)] == _brute(cur, ref, rng)
