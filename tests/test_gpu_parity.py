@@ -202,3 +202,13 @@ def test_intra_stage_by_tile_count(gpu_required, grid, qp):
     w, h = 32 * grid[0] + 21, 32 * grid[1] + 9
     cont, _, rec = encode_gen(w, h, 2, ebiv.synth_frame, intra=qp, gop=2, tiles=grid)
     _check(cont, w, h, rec)
+
+
+@pytest.mark.parametrize("w,h", [(16, 16), (48, 64), (64, 48), (80, 33), (135, 64), (193, 17)])
+@pytest.mark.parametrize("qp", [4, 20, 36])
+def test_prediction_at_the_planes_edges(gpu_required, w, h, qp):
+    """Moving clips whose rows end before, at and after a row of 64 bytes: eight samples are predicted from aligned
+    words only while these lie inside the row, and transforms of every size are coded."""
+    for gen in (ebiv.synth_pan, noisy_gen, flash_gen):
+        cont, _, rec = encode_gen(w, h, 5, gen, intra=qp, gop=5)
+        _check(cont, w, h, rec)
