@@ -3,14 +3,19 @@
 // loops of the encoder's rate-distortion search (every intra-mode trial and
 // every inter candidate transforms or Hadamard-scores its residual).
 //
-// One warp per block.  forwardDCT: lane l computes columns pass entries
-// tmp[k][j] = round(sum_i C[k][i] * src[i][j]) for k*n+j = l, l+32, ...
-// (int64 accumulation, rounding shift by 13, the int32 narrowing of the
-// reference), then row pass dst[k][m] = round(sum_j C[m][j] * tmp[k][j]);
-// the block, the intermediate and the DCT basis sit in shared memory.  satd:
-// the in-place Walsh-Hadamard butterflies of the rows, then the columns
-// (int32 arithmetic, wrapping as Go's does), and the sum of absolute values
-// (int64) as a warp reduction.
+// n threads per block, thread l with column l of the block in registers.
+// forwardDCT: tmp[k][l] = round(sum_i C[k][i] * src[i][l]) down the column,
+// then, through shared memory, row l: dst[l][m] = round(sum_j C[m][j] *
+// tmp[l][j]) (int64 accumulation, rounding shift by 13, the int32 narrowing of
+// the reference).  satd: the Walsh-Hadamard butterflies of the columns, then
+// the rows (int32 arithmetic, wrapping as Go's does, in which the order of the
+// two makes no difference), and the sum of absolute values (int64) as a
+// reduction over the block's threads.
+//
+// Bound by the block's 2 n^3 products, so nothing else is done per product:
+// the samples stay in registers and four words of the basis come with one load
+// that all threads share.  32,400 blocks of 8x8: 32 us with a warp per block,
+// a lane per output and two loads a product, 9 us now.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -23,71 +28,88 @@
 namespace ebiv {
 namespace dev {
 
-constexpr int kAnaWarps = 4;
+constexpr int kAnaThreads = 128;
 constexpr int kDCTScaleBits = 13;  // the DCT basis is scaled by 2^13 (ebiv/transform.go:15-40)
 
-__global__ void __launch_bounds__(32 * kAnaWarps) kAnalyze(const int32_t* __restrict__ src, int n, int count,
-                                                           const int32_t* __restrict__ basis, int32_t* __restrict__ dst,
-                                                           int64_t* __restrict__ satdOut) {
-  __shared__ int32_t sC[256];
-  __shared__ int32_t sBlk[kAnaWarps][256];
-  __shared__ int32_t sTmp[kAnaWarps][256];
-  const int nn = n * n;
-  for (int i = threadIdx.x; i < nn; i += blockDim.x) sC[i] = basis[i];
+// One output of a 1-D transform: row k of the basis with v.
+template <int N>
+__device__ __forceinline__ int32_t dctDot(const int4* c, int k, const int32_t (&v)[N]) {
+  int64_t acc = 1LL << (kDCTScaleBits - 1);
+#pragma unroll
+  for (int i = 0; i < N; i += 4) {
+    const int4 w = c[(k * N + i) / 4];
+    acc += (int64_t)w.x * v[i];
+    acc += (int64_t)w.y * v[i + 1];
+    acc += (int64_t)w.z * v[i + 2];
+    acc += (int64_t)w.w * v[i + 3];
+  }
+  return (int32_t)(acc >> kDCTScaleBits);
+}
+
+template <int N>
+__device__ __forceinline__ void hadamard(int32_t (&v)[N]) {
+#pragma unroll
+  for (int span = 1; span < N; span <<= 1)
+#pragma unroll
+    for (int a = 0; a < N; a++)
+      if (!(a & span)) {
+        const uint32_t x = (uint32_t)v[a], y = (uint32_t)v[a + span];
+        v[a] = (int32_t)(x + y);
+        v[a + span] = (int32_t)(x - y);
+      }
+}
+
+template <int N>
+__global__ void __launch_bounds__(kAnaThreads) kAnalyze(const int32_t* __restrict__ src, int count,
+                                                        const int32_t* __restrict__ basis, int32_t* __restrict__ dst,
+                                                        int64_t* __restrict__ satdOut) {
+  constexpr int kBlocks = kAnaThreads / N, kPitch = N + 1;
+  __shared__ int4 sC[N * N / 4];
+  __shared__ int32_t sTmp[kBlocks][N * kPitch];
+  if (threadIdx.x < N * N / 4) sC[threadIdx.x] = reinterpret_cast<const int4*>(basis)[threadIdx.x];
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blockIdx.x * kAnaWarps + warp;
-  if (b >= count) return;
-  const int32_t* s = src + (size_t)b * nn;
-  int32_t* blk = sBlk[warp];
-  int32_t* tmp = sTmp[warp];
-  for (int i = lane; i < nn; i += 32) blk[i] = s[i];
-  __syncwarp();
-  const int64_t round = 1LL << (kDCTScaleBits - 1);
+  const int l = threadIdx.x % N;
+  const size_t b = (size_t)blockIdx.x * kBlocks + threadIdx.x / N;
+  const bool mine = b < (size_t)count;  // every thread of a warp stays for its barriers
+  const int32_t* s = src + b * (N * N);
+  int32_t* tmp = sTmp[threadIdx.x / N];
+  int32_t v[N], t[N];
+#pragma unroll
+  for (int i = 0; i < N; i++) v[i] = mine ? s[i * N + l] : 0;
   if (dst) {
-    for (int o = lane; o < nn; o += 32) {
-      const int k = o / n, j = o - k * n;
-      int64_t acc = 0;
-      for (int i = 0; i < n; i++) acc += (int64_t)sC[k * n + i] * (int64_t)blk[i * n + j];
-      tmp[o] = (int32_t)((acc + round) >> kDCTScaleBits);
-    }
+#pragma unroll 8
+    for (int k = 0; k < N; k++) tmp[k * kPitch + l] = dctDot<N>(sC, k, v);
     __syncwarp();
-    int32_t* d = dst + (size_t)b * nn;
-    for (int o = lane; o < nn; o += 32) {
-      const int k = o / n, m = o - k * n;
-      int64_t acc = 0;
-      for (int j = 0; j < n; j++) acc += (int64_t)sC[m * n + j] * (int64_t)tmp[k * n + j];
-      d[o] = (int32_t)((acc + round) >> kDCTScaleBits);
+#pragma unroll
+    for (int j = 0; j < N; j++) t[j] = tmp[l * kPitch + j];
+    int4* const d = reinterpret_cast<int4*>(dst + b * (N * N) + l * N);
+#pragma unroll 2
+    for (int m = 0; m < N; m += 4) {
+      const int4 o = make_int4(dctDot<N>(sC, m, t), dctDot<N>(sC, m + 1, t), dctDot<N>(sC, m + 2, t), dctDot<N>(sC, m + 3, t));
+      if (mine) d[m / 4] = o;
     }
     __syncwarp();
   }
   if (satdOut) {
-    // Rows, then columns: one butterfly stage at a time over the whole
-    // block, each lane taking pairs (a, a + span) of the stage.
-    for (int pass = 0; pass < 2; pass++) {
-      for (int span = 1; span < n; span <<= 1) {
-        for (int q = lane; q < nn / 2; q += 32) {
-          // q-th pair of the stage: line (row or column) q / (n/2), pair q % (n/2) within it
-          const int line = q / (n / 2), p = q - line * (n / 2);
-          const int grp = p / span, off = p - grp * span;
-          const int a = grp * 2 * span + off, c = a + span;  // positions within the line
-          const int ia = pass == 0 ? line * n + a : a * n + line;
-          const int ic = pass == 0 ? line * n + c : c * n + line;
-          const int32_t x = blk[ia], y = blk[ic];
-          blk[ia] = (int32_t)((uint32_t)x + (uint32_t)y);
-          blk[ic] = (int32_t)((uint32_t)x - (uint32_t)y);
-        }
-        __syncwarp();
-      }
-    }
+    hadamard<N>(v);
+#pragma unroll
+    for (int i = 0; i < N; i++) tmp[i * kPitch + l] = v[i];
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < N; j++) t[j] = tmp[l * kPitch + j];
+    hadamard<N>(t);
     int64_t sum = 0;
-    for (int i = lane; i < nn; i += 32) {
-      const int32_t v = blk[i];
-      sum += v < 0 ? -(int64_t)v : (int64_t)v;
-    }
-    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (lane == 0) satdOut[b] = sum;
+#pragma unroll
+    for (int j = 0; j < N; j++) sum += t[j] < 0 ? -(int64_t)t[j] : (int64_t)t[j];
+    for (int o = N / 2; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (l == 0 && mine) satdOut[b] = sum;
   }
+}
+
+template <int N>
+static void launchAnalyze(const int32_t* src, int count, const int32_t* basis, int32_t* dst, int64_t* satd, cudaStream_t s) {
+  constexpr int kBlocks = kAnaThreads / N;
+  kAnalyze<N><<<(int)(((size_t)count + kBlocks - 1) / kBlocks), kAnaThreads, 0, s>>>(src, count, basis, dst, satd);
 }
 
 }  // namespace dev
@@ -160,8 +182,8 @@ int ebivgpu_fdct_satd(ebivgpu_analysis* a, const int32_t* residuals, int n, int 
   if (cudaMemcpyAsync(a->dSrc, residuals, (size_t)count * nn * 4, cudaMemcpyHostToDevice, a->stream) != cudaSuccess)
     return kErrDevice;
   cudaEventRecord(a->ev0, a->stream);
-  dev::kAnalyze<<<(count + dev::kAnaWarps - 1) / dev::kAnaWarps, 32 * dev::kAnaWarps, 0, a->stream>>>(
-      a->dSrc, n, count, a->dBasis + 256 * k, coeffs ? a->dDst : nullptr, satd ? a->dSatd : nullptr);
+  (n == 4 ? dev::launchAnalyze<4> : (n == 8 ? dev::launchAnalyze<8> : dev::launchAnalyze<16>))(
+      a->dSrc, count, a->dBasis + 256 * k, coeffs ? a->dDst : nullptr, satd ? a->dSatd : nullptr, a->stream);
   if (cudaGetLastError() != cudaSuccess) return kErrDevice;
   cudaEventRecord(a->ev1, a->stream);
   if ((coeffs && cudaMemcpyAsync(coeffs, a->dDst, (size_t)count * nn * 4, cudaMemcpyDeviceToHost, a->stream)) ||

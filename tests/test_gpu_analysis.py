@@ -25,3 +25,13 @@ def test_fdct_and_satd_match_the_oracle(gpu_required, n):
     blocks = rng.integers(-255, 256, size=(5, n, n), dtype=np.int64).astype(np.int32)
     assert a.fdct_satd(blocks, coeffs=False)[0] is None
     assert a.fdct_satd(blocks, satd=False)[1] is None
+
+
+@pytest.mark.parametrize("n", [4, 8, 16])
+@pytest.mark.parametrize("count", [1, 7, 8, 9, 31, 32, 33, 129])
+def test_batches_that_do_not_fill_their_last_group(gpu_required, n, count):
+    """Counts on both sides of the blocks that a group of 128 threads takes (32, 16 and 8)."""
+    blocks = np.random.default_rng(count).integers(-4080, 4081, size=(count, n, n), dtype=np.int64).astype(np.int32)
+    coef, s = ebiv.BlockAnalysis().fdct_satd(blocks)
+    assert (coef == transform_ref.forward_dct(blocks, n)).all()
+    assert (s == transform_ref.satd(blocks, n)).all()
