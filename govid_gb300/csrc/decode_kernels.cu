@@ -2203,6 +2203,8 @@ void launchEntropy(const FrameDesc* frames, const int4* jobs, int njobs, int* ne
 
 // The reconstruction launches overlap their start with the previous kernel
 // of the stream (programmatic dependent launch; the kernels wait for it).
+// A launch that is refused leaves its error for the caller's cudaGetLastError
+// (a round's is read when its results are collected).
 template <class... A>
 static void launchDependent(void (*k)(A...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};
@@ -2246,23 +2248,21 @@ static void launchIntraW(const FrameDesc* frames, const int2* jobs, int njobs, i
 void launchIntra(const FrameDesc* frames, const int2* jobs, int njobs, int maxTileMBs, int maxTileKeys, int warps,
                  cudaStream_t s) {
   if (njobs <= 0) return;
-  static int sms[64] = {0};
+  // Per device, once: the shared-memory limits of all three variants, and then
+  // the SM count, whose presence says that the limits are raised (engines of
+  // several threads may come here first together; each then raises them).
+  static std::atomic<int> sms[64];
   int d = 0;
   cudaGetDevice(&d);
-  bool first = false;
-  int nsm = 152;
-  if (d >= 0 && d < 64) {
-    if (!sms[d]) {
-      cudaDeviceGetAttribute(&sms[d], cudaDevAttrMultiProcessorCount, d);
-      sms[d] = std::max(1, sms[d]);
-      first = true;
-    }
-    nsm = sms[d];
-  }
-  if (first) {  // the shared-memory limits of all three, once per device
+  const bool known = d >= 0 && d < 64;
+  int nsm = known ? sms[d].load(std::memory_order_acquire) : 0;
+  if (!nsm) {
     allowIntraSmem<16>();
     allowIntraSmem<8>();
     allowIntraSmem<4>();
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, d);
+    nsm = std::max(1, nsm);
+    if (known) sms[d].store(nsm, std::memory_order_release);
   }
   const int flagMBs = std::max(1, std::min(maxTileMBs, dev::kIntraFlagMBs));
   int sortInts = std::max(0, maxTileMBs) + std::max(0, maxTileKeys);
