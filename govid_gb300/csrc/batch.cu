@@ -38,28 +38,28 @@ struct Slot {
   // per macroblock: whether its inter prediction waits for the previous
   // frame's intra stage; then two intra progress bytes (large tiles)
   uint8_t* dep = nullptr;
-  uint8_t* symLog = nullptr;   // the entropy stage's symbol log (symLogBytes)
-  uint32_t* symOff = nullptr;  // per macroblock: its first symbol in its tile's log
-  // One allocation, each part at a multiple of 256 bytes: with nine of them a
-  // slot the first pass of a new batch of 24 mixed streams takes 62 ms, with
-  // one 42 ms.
+  uint32_t* symOff = nullptr;  // per macroblock: the entries of its symbol log
+  // One allocation: with nine of them a slot the first pass of a new batch of
+  // 24 mixed streams takes 62 ms, with one 42 ms.  The parts lie one behind the
+  // other, those of larger words first, so that each is aligned and a slot
+  // takes exactly what its macroblocks need (the server admits by it).
   static size_t layout(size_t mbs, Slot* s, uint8_t* base) {
+    static_assert(sizeof(MBRec) % 16 == 0 && kCoefPerMB % 4 == 0 && sizeof(TileStat) % 16 == 0, "aligned parts");
     size_t at = 0;
     auto part = [&](auto** p, size_t n) {
       if (s) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(base + at);
-      at = al(at + n, 256);
+      at += n;
     };
     Slot none;
     Slot& d = s ? *s : none;
     part(&d.rec, mbs * sizeof(MBRec));
     part(&d.coef, mbs * kCoefPerMB * sizeof(uint32_t));
+    part(&d.ts, mbs * sizeof(TileStat));
+    part(&d.symOff, mbs * sizeof(uint32_t));
+    part(&d.intra, mbs * sizeof(uint32_t));
     part(&d.mv, mbs * 2 * sizeof(int16_t));
     part(&d.lv, mbs * sizeof(int16_t));
-    part(&d.intra, 2 * mbs * sizeof(uint32_t));
-    part(&d.ts, mbs * sizeof(TileStat));
     part(&d.dep, 3 * mbs);
-    part(&d.symLog, symLogBytes(mbs));
-    part(&d.symOff, mbs * sizeof(uint32_t));
     return at;
   }
   bool alloc(size_t mbs) {
@@ -953,9 +953,7 @@ int Engine::planRound(const std::vector<int>& ids, const std::vector<int>* maxFr
     fd.mvgrid = sl.mv;
     fd.lvgrid = sl.lv;
     fd.intraList = sl.intra;
-    fd.intraSorted = sl.intra + s.mbs;
     fd.tileStat = sl.ts;
-    fd.symLog = sl.symLog;
     fd.symOff = sl.symOff;
     fd.status = reinterpret_cast<int32_t*>(d + R.oStat) + di;
     fd.gate = gateDesc >= 0 ? reinterpret_cast<const int32_t*>(d + R.oStat) + gateDesc : nullptr;

@@ -587,6 +587,14 @@ __device__ __forceinline__ int decodeMB(WarpChain& d, int inter, MBRec* rec, uin
   return intra && w ? 1 : 0;
 }
 
+// A macroblock's log, and the same as 16-byte words: its coefficient region.
+constexpr int kLogEntries = kSymPerMB / 2, kLogWords = kSymPerMB / 16;
+static_assert(kSymPerMB % 16 == 0 && kHeaderEntries + blockEntries(16, 256) + kLastEntries <= kLogEntries,
+              "a macroblock's log");
+__device__ __forceinline__ uint32_t* coefRegion(const FrameDesc* fp, int idx) {
+  return fp->coef + (size_t)idx * kCoefPerMB;
+}
+
 // The full chain of a tile, by one warp (the frame's tables are in sT): the
 // rANS symbols drive the macroblock grammar, and every macroblock reached
 // gets its record (inter vectors as deltas), its coefficient regions and,
@@ -597,7 +605,6 @@ __device__ __noinline__ int fullChain(const FrameDesc* fp, int tile, const Entro
   const int mbCols = fp->mbCols;
   const int inter = fp->inter;
   MBRec* const recs = fp->mbrec;
-  uint32_t* const coefBase = fp->coef;
   const TileRange tr = fp->tiles[tile];
   uint32_t* const intraList = fp->intraList + tr.mbBase;
   const int x0 = tr.mbX0, x1 = tr.mbX1, y0 = tr.mbY0, y1 = tr.mbY1;
@@ -608,7 +615,7 @@ __device__ __noinline__ int fullChain(const FrameDesc* fp, int tile, const Entro
   for (int mby = y0; mby < y1 && !d.err; mby++) {
     for (int mbx = x0; mbx < x1; mbx++) {
       const int idx = mby * mbCols + mbx;
-      if (decodeMB(d, inter, recs + idx, coefBase + (size_t)idx * kCoefPerMB, lane)) {
+      if (decodeMB(d, inter, recs + idx, coefRegion(fp, idx), lane)) {
         if (lane == 0) intraList[intraCount] = (uint32_t)idx;
         intraCount++;
       }
@@ -634,27 +641,16 @@ __device__ __noinline__ int fullChain(const FrameDesc* fp, int tile, const Entro
   return done;
 }
 
-// A tile's log and its size in entries: kSymPerMB bytes per macroblock, and
-// for the frame's first tiles room for a macroblock more (the chain reserves
-// that much before each, so that a tile of few macroblocks can use all of its
-// own).
-__device__ __forceinline__ uint16_t* tileLog(const FrameDesc* fp, const TileRange& tr, int tile, int* entries) {
-  static_assert(kSpareLogBytes >= 2 * kMBEntries && kSpareLogBytes % 16 == 0, "spare room of a tile's log");
-  const int total = (tr.mbX1 - tr.mbX0) * (tr.mbY1 - tr.mbY0);
-  *entries = (total * kSymPerMB + (tile < kSpareLogTiles ? kSpareLogBytes : 0)) / 2;
-  return reinterpret_cast<uint16_t*>(fp->symLog + (size_t)tr.mbBase * kSymPerMB +
-                                     (size_t)min(tile, kSpareLogTiles) * kSpareLogBytes);
-}
-
 // The symbol chain of a tile, by one thread (Chain); false when it leaves the
 // tile to the full chain.
 __device__ __forceinline__ bool symbolChain(const FrameDesc* fp, int tile, const EntropyTables& sT) {
   const TileRange tr = fp->tiles[tile];
-  const int total = (tr.mbX1 - tr.mbX0) * (tr.mbY1 - tr.mbY0);
-  int cap;
-  uint16_t* const log = tileLog(fp, tr, tile, &cap);
+  const int tw = tr.mbX1 - tr.mbX0, total = tw * (tr.mbY1 - tr.mbY0);
+  uint16_t* const log = reinterpret_cast<uint16_t*>(coefRegion(fp, tr.mbY0 * fp->mbCols + tr.mbX0));
   Chain d;
-  if (!d.run(fp->pkt + tr.offset, tr.length, sT, fp->inter, total, log, cap, fp->symOff + tr.mbBase)) return false;
+  if (!d.run(fp->pkt + tr.offset, tr.length, sT, fp->inter, total, log, kLogEntries, fp->symOff + tr.mbBase, tw,
+             fp->mbCols))
+    return false;
   TileStat* ts = fp->tileStat + tile;
   ts->err = 0;
   ts->done = total;
@@ -664,8 +660,8 @@ __device__ __forceinline__ bool symbolChain(const FrameDesc* fp, int tile, const
 
 // Entropy jobs: up to kEntropyWarps tiles of one frame per job, one warp per
 // tile, sharing the frame's symbol tables.  A tile runs the symbol chain
-// when its frame has a symbol log (the full chain when the log would
-// overflow), else the full chain.  With a queue counter the grid is
+// when its frame has a symbol log (the full chain when it leaves the tile),
+// else the full chain.  With a queue counter the grid is
 // persistent: each CTA takes jobs (longest first, as listed) until none are
 // left, so a round with more jobs than resident CTAs has no second-wave
 // tail; without one, CTA b runs job b.
@@ -686,7 +682,7 @@ __global__ void __launch_bounds__(32 * kEntropyWarps, 2) kEntropy(const FrameDes
     if (warp < job.z) {
       const int tile = job.y + warp;
       bool done = false;
-      if (fp->symLog) {
+      if (fp->symOff) {
         const TileRange tr = fp->tiles[tile];
         const int mbs = (tr.mbX1 - tr.mbX0) * (tr.mbY1 - tr.mbY0);
         for (int k = lane; k < mbs; k += 32) fp->symOff[tr.mbBase + k] = kSkipOffset;
@@ -705,11 +701,13 @@ __global__ void __launch_bounds__(32 * kEntropyWarps, 2) kEntropy(const FrameDes
 // per macroblock over every macroblock of the launch's tiles (grid.x: job *
 // kEntropyTilesPerJob + tile within the job; grid.y * kParseWarps: the
 // macroblock's raster index within its tile).  A skip macroblock's record is
-// fixed; of another one the whole warp reads the header, and then each lane
-// one log entry at a time of its blocks: the entries name their kind, so a
-// lane finds its block, its position and its place among the block's levels
-// by counting the ends and tokens before it.  A flag per macroblock marks the
-// intra ones for kTileFinish.
+// fixed; of another one the warp takes the log out of the macroblock's
+// coefficient region into shared memory, whole, before it writes levels there;
+// then all of it reads the header, and each lane one log entry at a time of
+// its blocks: the entries name their kind, so a lane finds its block, its
+// position and its place among the block's levels by counting the ends and
+// tokens before it.  A flag per macroblock marks the intra ones for
+// kTileFinish.
 constexpr int kParseWarps = 8;
 
 struct ParseBlocks {
@@ -717,10 +715,10 @@ struct ParseBlocks {
   uint32_t cmode;  // the chroma intra mode
 };
 
-// The blocks of plan p whose entries start at entry `from` of the 32 entries
-// at log index `off` (lane's entry of them: v); nothing at or past `end` is
-// read.  Levels go to coef, luma modes to lmode (shared memory).
-__device__ __forceinline__ ParseBlocks parseBlocks(const uint16_t* log, int off, int end, int from, uint32_t v,
+// The blocks of plan p whose entries start at entry `from` of the log's first
+// 32 (lane's entry of them: v); the log has `end` entries.  Levels go to coef,
+// luma modes to lmode (log and lmode in shared memory).
+__device__ __forceinline__ ParseBlocks parseBlocks(const uint16_t* log, int end, int from, uint32_t v,
                                                    const BlockPlan& p, uint32_t* coef, uint8_t* lmode, int lane) {
   ParseBlocks out = {0u, 0u};
   const int blocks = p.nLuma + (p.cb ? 1 : 0) + (p.cr ? 1 : 0);
@@ -730,7 +728,7 @@ __device__ __forceinline__ ParseBlocks parseBlocks(const uint16_t* log, int off,
   // The block that is open at the start of a pass: its tokens and nonzero ones
   // so far, the first one's position and magnitude, the last one's position
   // and the parity of the magnitudes.
-  int done = 0, openTokens = 0, openCount = 0, openFirst = 0, openMag = 0, openLast = 0, openOdd = 0;
+  int off = 0, done = 0, openTokens = 0, openCount = 0, openFirst = 0, openMag = 0, openLast = 0, openOdd = 0;
   while (done < blocks) {
     const uint32_t kind = v & kLogKind;
     const int sym = (int)((v >> kLogShift) & 7u);
@@ -825,6 +823,7 @@ __device__ __forceinline__ ParseBlocks parseBlocks(const uint16_t* log, int off,
 
 __global__ void __launch_bounds__(32 * kParseWarps) kParseMB(const FrameDesc* frames, const int4* jobs, int njobs) {
   __shared__ __align__(16) uint8_t sMode[kParseWarps][16];
+  __shared__ uint4 sLog[kParseWarps][kLogWords];
   const int jb = (int)blockIdx.x / kEntropyTilesPerJob, tj = (int)blockIdx.x % kEntropyTilesPerJob;
   if (jb >= njobs) return;
   const int4 job = jobs[jb];
@@ -840,15 +839,19 @@ __global__ void __launch_bounds__(32 * kParseWarps) kParseMB(const FrameDesc* fr
   const int idx = (tr.mbY0 + k / tw) * fp->mbCols + tr.mbX0 + k % tw;
   uint4* const words = reinterpret_cast<uint4*>(fp->mbrec + idx);
   uint8_t* const flags = reinterpret_cast<uint8_t*>(fp->lvgrid) + tr.mbBase;
-  const uint32_t off = fp->symOff[tr.mbBase + k];
-  if (off == kSkipOffset) {
+  const uint32_t entries = fp->symOff[tr.mbBase + k];
+  if (entries == kSkipOffset) {
     if (lane < 3) words[lane] = make_uint4(lane ? 0u : (uint32_t)kRecSkip, 0u, 0u, lane == 2 ? kWriteAll : 0u);
     if (lane == 0) flags[k] = 0;
     return;
   }
-  int end;
-  const uint16_t* const log = tileLog(fp, tr, tile, &end);
-  const uint32_t v = (int)off + lane < end ? (uint32_t)log[off + lane] : 0u;
+  uint32_t* const coef = coefRegion(fp, idx);
+  const int end = (int)min(entries, (uint32_t)kLogEntries);
+  const uint4* const from = reinterpret_cast<const uint4*>(coef);
+  for (int i = lane; 8 * i < end; i += 32) sLog[warp][i] = from[i];
+  __syncwarp();
+  const uint16_t* const log = reinterpret_cast<const uint16_t*>(sLog[warp]);
+  const uint32_t v = lane < end ? (uint32_t)log[lane] : 0u;
   int n = 0;
   auto next = [&]() -> uint32_t { return (__shfl_sync(kFull, v, n++) >> kLogShift) & 255u; };
   auto value = [&]() -> uint32_t {
@@ -883,7 +886,7 @@ __global__ void __launch_bounds__(32 * kParseWarps) kParseMB(const FrameDesc* fr
   uint8_t* const lmode = sMode[warp];
   if (lane < 4) reinterpret_cast<uint32_t*>(lmode)[lane] = 0;
   __syncwarp();
-  const ParseBlocks b = parseBlocks(log, (int)off, end, n, v, p, fp->coef + (size_t)idx * kCoefPerMB, lmode, lane);
+  const ParseBlocks b = parseBlocks(log, end, n, v, p, coef, lmode, lane);
   __syncwarp();
   if (lane < 3) {
     // Every block is there, so all of the macroblock is written (of an intra

@@ -48,18 +48,13 @@ constexpr uint32_t kWriteAll = 0x3FFFFu;
 // int4{descriptor, first tile, tile count, 0}.
 constexpr int kEntropyTilesPerJob = 4;
 
-// Bytes of symbol log per macroblock in a decode slot (the entropy stage's
-// symbol path; a tile whose symbols do not fit takes the full chain, which
-// decodes it a second time).  Key frames coded at q18 average about 125
-// symbols of two bytes per macroblock, small textured ones at q22 185, and the
-// chain also reserves room for a whole block before decoding it, so the log
-// holds 256 symbols.
-constexpr int kSymPerMB = 512;
-// The first tiles of a frame have room for one more macroblock's most symbols
-// each (a frame of more tiles is cut into tiles of many macroblocks, or is
-// decoded by the full chain).
-constexpr int kSpareLogTiles = 64, kSpareLogBytes = 3232;
-constexpr size_t symLogBytes(size_t mbs) { return mbs * kSymPerMB + (size_t)kSpareLogTiles * kSpareLogBytes; }
+// Bytes of symbol log per macroblock: the entropy stage logs a macroblock's
+// symbols in its coefficient region, from where kParseMB reads them all before
+// it writes the levels there, so the log takes no memory of its own.  816
+// entries of two bytes: key frames coded at q18 average about 125 a macroblock,
+// small textured ones at q22 185; 384 nonzero coefficients without an escape
+// take 843.
+constexpr int kSymPerMB = 4 * kCoefPerMB;
 
 struct TileStat {
   int32_t err;         // 0 or an ebiv status
@@ -91,9 +86,8 @@ struct FrameDesc {
   MBRec* mbrec;
   uint32_t* coef;
   int16_t* mvgrid;      // 2 x int16 per macroblock (wide-tile fallback rows)
-  int16_t* lvgrid;      // 1 x int16 per macroblock (wide-tile fallback rows)
+  int16_t* lvgrid;      // per macroblock one byte: intra and written (kParseMB)
   uint32_t* intraList;  // per tile at mbBase: intra macroblocks, raster order
-  uint32_t* intraSorted;// per tile at mbBase: the same grouped by level
   TileStat* tileStat;
   int32_t* status;      // frame status, written by the commit step
   // Status of the frame this one depends on (the previous frame of the
@@ -109,10 +103,9 @@ struct FrameDesc {
   int32_t prevKey;
   int32_t pad2;
   uint8_t* dep;
-  // Symbol path of the entropy stage (null symLog: every tile takes the full
-  // chain): the tiles' logs (symLogBytes), and per macroblock the index of its
-  // first symbol in its tile's log (at mbBase + raster index within the tile).
-  uint8_t* symLog;
+  // Symbol path of the entropy stage (null: every tile takes the full chain):
+  // per macroblock the entries of its log (at mbBase + raster index within the
+  // tile).
   uint32_t* symOff;
 };
 

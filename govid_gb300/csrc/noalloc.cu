@@ -58,14 +58,15 @@ constexpr size_t kOffIntra = a256(kOffLV + (size_t)kNAMaxMBs * sizeof(int16_t));
 constexpr size_t kOffTS = a256(kOffIntra + 2 * (size_t)kNAMaxMBs * sizeof(uint32_t));
 constexpr size_t kOffPkt = a256(kOffTS + (size_t)kNAMaxMBs * sizeof(TileStat));
 constexpr size_t kNABytes = a256(kOffPkt + kNAMaxPacket);
-static_assert(kNABytes == EBIVGPU_NOALLOC_SCRATCH_BYTES, "the header states the scratch size");
-static_assert(kNABytes < (16u << 20), "the no-allocation scratch stays modest");
+// The header's figure is part of the interface; the layout fits it.
+static_assert(kNABytes <= EBIVGPU_NOALLOC_SCRATCH_BYTES && EBIVGPU_NOALLOC_SCRATCH_BYTES - kNABytes < 4096,
+              "the header states the scratch size");
 
 }  // namespace
 }  // namespace ebiv
 
 // The scratch: one per device, in the module's static device memory.
-static __device__ __align__(256) unsigned char gNoAllocScratch[ebiv::kNABytes];
+static __device__ __align__(256) unsigned char gNoAllocScratch[EBIVGPU_NOALLOC_SCRATCH_BYTES];
 
 namespace ebiv {
 namespace {
@@ -117,7 +118,6 @@ void fillDesc(FrameDesc& fd, uint8_t* d, int which, const Geometry& g, const Pay
   fd.mvgrid = reinterpret_cast<int16_t*>(d + kOffMV);
   fd.lvgrid = reinterpret_cast<int16_t*>(d + kOffLV);
   fd.intraList = reinterpret_cast<uint32_t*>(d + kOffIntra);
-  fd.intraSorted = fd.intraList + (size_t)g.mbCols * g.mbRows;
   fd.tileStat = reinterpret_cast<TileStat*>(d + kOffTS);
   fd.status = reinterpret_cast<int32_t*>(d + kOffStatus) + which;
   fd.gate = nullptr;

@@ -104,12 +104,16 @@ EBIV_DEV uint32_t rowOf(int c) {
 constexpr uint32_t kLogToken = 0, kLogSign = 1u << 6, kLogMode = 2u << 6, kLogValue = 3u << 6, kLogKind = 3u << 6;
 constexpr int kLogShift = 8;
 constexpr uint32_t kLogNonzero = 4;               // token flag, where Chain::far looks
-constexpr uint32_t kSkipOffset = 0xFFFFFFFFu;     // the offset of a skip macroblock: it has no log
-// The most entries of a macroblock: the header (mode, reference, partition,
-// eight vector components, pattern, transform size), four for a coefficient
-// (token, escape value and sign), the mode, end and last sign of 18 blocks,
-// and the four that are written ahead.
-constexpr int kMBEntries = 5 + 8 * 2 + 4 * 384 + 18 * 3 + 4;
+constexpr uint32_t kSkipOffset = 0xFFFFFFFFu;     // a skip macroblock: it has no log
+// The entries of a macroblock's header (mode, reference, partition, eight
+// vector components, pattern, transform size), the most that n blocks with
+// `coefs` coefficients take without escapes (a token and a sign for each
+// coefficient, the mode, end and last sign of each block) and what an escape
+// adds (its value).  The most of a macroblock are all of these together.
+constexpr int kHeaderEntries = 5 + 8 * 2, kEscapeEntries = 2;
+EBIV_DEV constexpr int blockEntries(int n, int coefs) { return 3 * n + 2 * coefs; }
+constexpr int kLastEntries = 4;  // kept free: the next macroblock's transform size, once
+constexpr int kMBEntries = kHeaderEntries + 3 * 18 + (2 + kEscapeEntries) * 384 + kLastEntries;
 
 // The entry of symbol s of context c, which starts at st and has frequency
 // freq, in a row that keeps class cls (signs).
@@ -194,8 +198,16 @@ struct Chain {
   const uint32_t* wp;
   int32_t rem;
   const EntropyTables* t;
-  uint16_t* log;   // the tile's log
-  uint16_t* lp;    // its next entry
+  // The log.  With width 0 the entries of all macroblocks follow one another;
+  // else each macroblock has `pitch` of its own, the tile's rows (of `width`)
+  // lie `gap` more than theirs apart, and log moves on by that with the rows:
+  // macroblock mb, before rowEnd, has those from log + mb * pitch.  room: what
+  // the macroblock has left when its open kind of blocks takes the most.
+  uint16_t* log;
+  uint16_t* lp;     // the next entry
+  uint16_t* first;  // the macroblock's first one
+  uint16_t* end;    // the end of what it, or the tile, has
+  int32_t width, pitch, gap, rowEnd, room;
   int32_t stop;    // macroblocks to decode; 0 after a failure
   // The grammar inside a macroblock's blocks.  kind: its block entry; left:
   // the blocks after this one that have the same, -1 past the macroblock's
@@ -208,11 +220,12 @@ struct Chain {
   // position after the first nonzero token's and before this one (unary, the
   // oldest lost).  far: bit 2 is set once a nonzero token was kSDHMinSpan or
   // more positions after the first.
-  // The macroblocks: mb is the current one, mbOff their offsets, cap the
-  // log's size; intraOnly: no mode in front of a macroblock.
+  // The macroblocks: mb is the current one, mbOff where their logs begin
+  // (width 0) or how many entries they have; intraOnly: no mode in front of a
+  // macroblock.
   uint4 kind;
   int32_t left;
-  int32_t mb, cap;
+  int32_t mb;
   bool intraOnly;
   uint32_t* mbOff;
   uint32_t queue, z, bands, seen, since, far;
@@ -235,8 +248,22 @@ struct Chain {
     put(kLogValue | (v & 255u) << kLogShift);
   }
   // A symbol that cannot be decoded (an unused context, a byte before the
-  // tile's first): the tile is left to the full chain.
+  // tile's first), or one with no room: the tile is left to the full chain.
   EBIV_DEV void fail() { stop = 0; }
+  // The log's part for macroblock mb, from lp on with width 0.
+  EBIV_DEV void open() {
+    if (width) {
+      while (mb >= rowEnd) {
+        rowEnd += width;
+        log += gap;
+      }
+      lp = log + (ptrdiff_t)mb * pitch;
+      end = lp + pitch;
+    }
+    first = lp;
+  }
+  // All of macroblock mb is in the log.
+  EBIV_DEV void close() { mbOff[mb] = (uint32_t)(width ? lp - first : first - log); }
   // Keeps off below 32.
   EBIV_DEV void refill() {
 #ifdef __CUDACC__  // without a branch
@@ -350,40 +377,52 @@ struct Chain {
     bands = __funnelshift_r(bands, 0u, adv);
   }
 
-  // The blocks of the queue's next byte.
-  EBIV_DEV void nextKind() {
+  // The blocks of the queue's next byte, when the log has room for them behind
+  // the entry lp[j].
+  EBIV_DEV void nextKind(int j) {
     kind = entryAt((uint32_t)offsetof(EntropyTables, block) - 16 + 16 * (queue & 15u));
     left = (int32_t)((queue >> 4) & 15u);
+    const int most = (queue & 3u) != 0 ? blockEntries(left + 1, 256) : blockEntries(left + 1, 64 * (left + 1));
     queue >>= 8;
+    room = (int32_t)(end - lp) - (j + 1) - most - kLastEntries;
+    if (room < 0) {
+      fail();
+      left = -1;
+    }
   }
   // The blocks of an intra macroblock of transform size tx.
   static EBIV_DEV uint32_t intraQueue(uint32_t tx) {
     return (tx + 5u) | ((16u >> (2 * tx)) - 1) << 4 | (8u | 4u << 8) << 8;
   }
   // After the last block of a kind: the next kind; in a frame of intra
-  // macroblocks only, the next one's transform size and then its blocks (e is
-  // the symbol of log index `at`).
-  EBIV_DEV void endedKind(const uint4& e, int at) {
+  // macroblocks only, the next one's transform size, which is the first entry
+  // of its log, and then its blocks (e is the symbol of lp[j]).
+  EBIV_DEV void endedKind(const uint4& e, int j) {
     if ((e.w & kLogKind) == kLogValue) {
       queue = intraQueue(min((e.w >> kLogShift) & 15u, 2u));  // alphabet size 3
-      mbOff[++mb] = (uint32_t)at;
+      lp += j;
+      close();
+      mb++;
+      open();
+      *lp = (uint16_t)e.w;
+      lp -= j;
     } else if (queue == 0) {
-      if (!intraOnly || mb + 1 >= stop || at + 1 + kMBEntries > cap) return;
+      if (!intraOnly || mb + 1 >= stop) return;
       kind = make_uint4(rowOf(ctxTxSize), 0u, 0u, 0u);
       left = 0;
       return;
     }
-    nextKind();
+    nextKind(j);
   }
   // The grammar after a block's end, its last sign, or a transform size (the
-  // symbol of entry e, of log index `at`): the offset of the next symbol,
-  // which state xn decodes.
-  EBIV_DEV uint32_t ended(const uint4& e, int at, uint32_t xn) {
+  // symbol of entry e, at lp[j]): the offset of the next symbol, which state
+  // xn decodes.
+  EBIV_DEV uint32_t ended(const uint4& e, int j, uint32_t xn) {
     const bool sign = (seen & kGroupMask) != 0 && !(far & kLogNonzero);
     seen = kClassMask;
     since = far = 0;
     left -= sign ? 0 : 1;
-    if (left < 0) endedKind(e, at);
+    if (left < 0) endedKind(e, j);
     z = left < 0 ? 1u << 31 : kind.y;
     bands = kind.z;
     return (sign ? kLastSignRow : kind.x) | (xn & kBucketMask);
@@ -391,10 +430,11 @@ struct Chain {
 
   // The symbols of a macroblock's blocks (decodeBlock, ebiv/residual.go:79-126),
   // which `blocks` lists as `queue` does, and with intraOnly those of the
-  // macroblocks after it while the log has room for the most they can take.
+  // macroblocks after it.
   EBIV_DEV void tokens(uint32_t blocks) {
     queue = blocks;
-    nextKind();
+    nextKind(-1);
+    if (left < 0) return;
     z = kind.y;
     bands = kind.z;
     seen = kClassMask;
@@ -429,7 +469,7 @@ struct Chain {
 #define EBIV_STUB(J, X, XN, E, F)                                                             \
   if ((int32_t)(E.z << 4 & ~(z | small1)) < 0) { /* kEBlock */                                \
     EBIV_UPDATE(J, X, E)                                                                      \
-    F = entryAt(ended(E, count() + J, XN));                                                   \
+    F = entryAt(ended(E, J, XN));                                                             \
   } else {                                                                                    \
     n = J;                                                                                    \
     if ((int32_t)(z | small1) < 0 || !(E.z & kEImpure)) goto stopped;                         \
@@ -513,18 +553,20 @@ struct Chain {
           bands = 1u << 12;
         } else {
           put(tEOB << kLogShift);
-          e = entryAt(ended(make_uint4(0u, 0u, 0u, 0u), count() - 1, x0));
+          e = entryAt(ended(make_uint4(0u, 0u, 0u, 0u), -1, x0));
           if (left < 0) return;
         }
       } else if (e.z & kEBlock) {
         e = symbolOf(e);
         put(e.w);
-        e = entryAt(ended(e, count() - 1, x0));
+        e = entryAt(ended(e, -1, x0));
         if (left < 0) return;
       } else if ((e.z & (kEUnused | kEEnd)) != 0) {
         // A failure, or an escape: its value, then the sign unless it is the
         // first nonzero token.
         e = symbolOf(e);
+        room -= kEscapeEntries;
+        if (room < 0) return fail();
         put(e.w);
         putValue(classValue(ctxEscClass));
         if (seen & kGroupMask) put(kLogSign | sym(ctxSign) << kLogShift);
@@ -619,16 +661,21 @@ struct Chain {
     return true;
   }
 
-  // The chain of a tile: len bytes at buf, total macroblocks, its log into
-  // tileLog (cap entries) and the first log entry of each macroblock that is
-  // not skip into mbOff (which holds kSkipOffset everywhere before).  False
-  // when the tile is left to the full chain: a symbol failed, or the log would
-  // overflow (before a macroblock there must be room for the most entries it
-  // can take).
+  // The chain of a tile: len bytes at buf, total macroblocks.  Its log goes
+  // into tileLog, which has `entries` entries, or with a tile width as many for
+  // each macroblock of a frame `stride` macroblocks wide, of which tileLog
+  // holds the tile's first.  offsets (kSkipOffset everywhere before) gets the
+  // first entry of each macroblock that is not skip, with a tile width the
+  // number of its entries.  False when the tile is left to the full chain: a
+  // symbol failed, or there was no room for the most entries that could
+  // follow.
   EBIV_DEV bool run(const uint8_t* buf, uint32_t len, const EntropyTables& tables, int inter, int total,
-                    uint16_t* tileLog, int entries, uint32_t* offsets) {
+                    uint16_t* tileLog, int entries, uint32_t* offsets, int tileWidth = 0, int stride = 0) {
     log = lp = tileLog;
-    cap = entries;
+    end = log + entries;
+    pitch = entries;
+    width = rowEnd = tileWidth;
+    gap = (stride - tileWidth) * entries;
     mbOff = offsets;
     stop = total;
     intraOnly = !inter;
@@ -640,8 +687,8 @@ struct Chain {
         mode = skips(mb, &mb);
         if (mode == mbSkip) break;
       }
-      if (count() + kMBEntries > cap) return false;
-      mbOff[mb] = (uint32_t)count();
+      open();
+      if (end - lp < kHeaderEntries + kLastEntries) return false;
       if (inter) put(kLogValue | mode << kLogShift);
       uint32_t cbp = kNumCBP - 1;
       if (mode != mbIntra) {
@@ -666,6 +713,8 @@ struct Chain {
       if (chroma) blocks |= (4u | (chroma - 1) << 4) << (cbp & cbpLuma ? 8 : 0);
       if (mode == mbIntra) blocks = intraQueue(tx);
       if (blocks != 0 && stop != 0) tokens(blocks);
+      if (stop == 0) return false;
+      close();
     }
     return stop == total;
   }
