@@ -34,9 +34,9 @@ namespace dev {
 constexpr unsigned kFull = 0xffffffffu;
 
 // Per transform size and scan position: row-major index (bits 0-7) and the
-// offset of the position's band in the symbol-table rows,
-// bandOf(i) * kNumPrevClass * 64 (bits 8-19).  One entry past each scan is
-// zero, so the next position's entry can always be loaded.
+// offset of the position's band in the symbol-table rows, bandOf(i) *
+// kGroupBytes (from bit 8).  One entry past each scan is zero, so the next
+// position's entry can always be loaded.
 __constant__ uint32_t cScanRow[3][257];
 // The same positions for lanes that read different ones.
 __device__ uint8_t gScan[3][256];
@@ -120,18 +120,21 @@ struct WarpChain {
     return 0;
   }
 
-  // The next symbol of context row / 64.
-  __device__ __forceinline__ int symAt(int row) {
+  __device__ __forceinline__ uint4 entryAt(uint32_t offset) const {
+    return *reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(t->entry) + offset);
+  }
+  // The next symbol of the context at a row (rowOf).
+  __device__ __forceinline__ int symAt(uint32_t row) {
     if (err) return 0;
     const uint32_t x = x0;
-    const uint32_t slot = x & (kM - 1);
-    const uint4* e = t->entry + rowOf(row >> 6) / 16 + (slot >> 6) * 4;
-    if (e->z & kEUnused) return fail(kErrCorrupt);  // symbol decoded from an unused context
-    if (e->z & kEImpure) {
-      e = t->entry + e->y;
-      while (slot >= e[1].y) e++;
+    uint4 e = entryAt(row | (x & kBucketMask));
+    if (e.z & (kEImpure | kEUnused)) {
+      if (e.z & kEUnused) return fail(kErrCorrupt);  // symbol decoded from an unused context
+      uint32_t q = 16 * e.y;
+      e = entryAt(q);
+      for (uint4 n = entryAt(q += 16); (x & (kM - 1)) >= n.y; n = entryAt(q += 16)) e = n;
     }
-    uint32_t xn = e->x * (x >> kScaleBits) + x - e->y;
+    uint32_t xn = e.x * (x >> kScaleBits) + x - e.y;
     if (xn < kLower) {
       if (pos >= 2 && xn >= (kLower >> 16)) {
         if (xn < (kLower >> 8)) {  // two bytes
@@ -159,9 +162,9 @@ struct WarpChain {
     x1 = x2;
     x2 = x3;
     x3 = xn;
-    return (int)((e->w >> kLogShift) & (row < ctxTokenBase << 6 ? 15u : 7u));
+    return (int)((e.w >> kLogShift) & 15u);
   }
-  __device__ __forceinline__ int sym(int ctx) { return symAt(ctx << 6); }
+  __device__ __forceinline__ int sym(int ctx) { return symAt(rowOf(ctx)); }
   // Initialises the four states from the end of the tile's bytes
   // (ransDecoder.reset, ebiv/rans.go:236-250); false when the stream is too short.
   __device__ __forceinline__ bool reset(const uint8_t* b, uint32_t len, const EntropyTables* tables) {
@@ -200,21 +203,21 @@ __device__ __forceinline__ int unzigzag(uint32_t u) { return (int)(u >> 1) ^ -(i
 __device__ __forceinline__ int mvComponent(WarpChain& d, int classCtx) { return unzigzag(classValue(d, classCtx)); }
 
 // decodeBlock (ebiv/residual.go:79-126): the block's nonzero levels are
-// written as packed entries after a count word (by lane 0).  row is the entry
-// row of the block's token contexts at band 0 and previous class 0 (context *
-// 64); the band and previous class add their row offsets.  Returns the count.
-__device__ __forceinline__ int entropyBlock(WarpChain& d, int row, int sz, uint32_t* region, int lane) {
+// written as packed entries after a count word (by lane 0).  row is the row of
+// the block's token contexts at band 0 and previous class 0; the band and
+// previous class add their offsets.  Returns the count.
+__device__ __forceinline__ int entropyBlock(WarpChain& d, uint32_t row, int sz, uint32_t* region, int lane) {
   const uint32_t* sb = cScanRow[sz];
   const int total = 16 << (2 * sz);
   int first = -1, last = -1, count = 0;
   int32_t sumAbs = 0;
-  int pc = 0;  // previous class * 64
+  uint32_t pc = 0;  // previous class * kClassBytes
   uint32_t firstPos = 0;
   int32_t firstMag = 0;
   uint32_t cur = sb[0];
   for (int i = 0; i < total; i++) {
     const uint32_t nxt = sb[i + 1];  // next position's entry, loaded early (the table is padded)
-    const int t = d.symAt(row + (int)(cur >> 8) + pc);
+    const int t = d.symAt(row + (cur >> 8) + pc);
     if (t == tEOB) break;
     if (t == tZero) {
       pc = 0;
@@ -224,10 +227,10 @@ __device__ __forceinline__ int entropyBlock(WarpChain& d, int row, int sz, uint3
     int mag;
     if (t == tEscape) {
       mag = 5 + (int)classValue(d, ctxEscClass);
-      pc = 2 * 64;
+      pc = 2 * kClassBytes;
     } else {
       mag = t;
-      pc = t == tOne ? 64 : 2 * 64;
+      pc = t == tOne ? kClassBytes : 2 * kClassBytes;
     }
     sumAbs = wadd(sumAbs, mag);
     const uint32_t pos = cur & 0xFFu;
@@ -236,7 +239,7 @@ __device__ __forceinline__ int entropyBlock(WarpChain& d, int row, int sz, uint3
       firstPos = pos;
       firstMag = mag;
     } else {
-      if (d.symAt(ctxSign << 6) == 1) mag = -mag;
+      if (d.sym(ctxSign) == 1) mag = -mag;
       if (lane == 0) region[1 + count] = pos | ((uint32_t)mag << 8);
     }
     count++;
@@ -244,7 +247,7 @@ __device__ __forceinline__ int entropyBlock(WarpChain& d, int row, int sz, uint3
     cur = nxt;
   }
   if (first >= 0) {
-    const bool neg = (last - first >= kSDHMinSpan) ? (sumAbs & 1) == 1 : d.symAt(ctxSign << 6) == 1;
+    const bool neg = (last - first >= kSDHMinSpan) ? (sumAbs & 1) == 1 : d.sym(ctxSign) == 1;
     if (lane == 0) region[1] = firstPos | ((uint32_t)(neg ? -firstMag : firstMag) << 8);
   }
   if (lane == 0) region[0] = (uint32_t)count;
@@ -328,12 +331,13 @@ __device__ __forceinline__ int entropyBlocks(WarpChain& d, Rec& r, const BlockPl
                                              uint32_t* nzOut) {
   const int nEnt = p.nLuma + (p.cb ? 1 : 0) + (p.cr ? 1 : 0);
   const int bw = (16 << (2 * p.tx)) + 1;  // words per luma block region
-  const int lumaRow = (ctxTokenBase + p.tx * kNumBands * kNumPrevClass) << 6;
+  const uint32_t lumaRow = (uint32_t)(p.tx * kNumBands) * kGroupBytes;
   int done = 0;
   uint32_t nz = 0;
 #pragma unroll 1
   for (int e = 0; e < nEnt; e++) {
-    int row, sz;
+    uint32_t row;
+    int sz;
     uint32_t* region;
     uint32_t bit;
     if (e < p.nLuma) {
@@ -346,7 +350,7 @@ __device__ __forceinline__ int entropyBlocks(WarpChain& d, Rec& r, const BlockPl
       sz = 1;
       const bool isCb = p.cb && e == p.nLuma;
       if (isCb && p.intra) r.w1 |= (uint32_t)d.sym(ctxChromaMode) << 8;
-      row = (ctxTokenBase + kLumaTokenCtx) << 6;
+      row = rowOf(ctxTokenBase + kLumaTokenCtx);
       region = coef + (isCb ? kCoefCb : kCoefCr);
       bit = isCb ? (1u << 16) : (1u << 17);
     }
@@ -2169,7 +2173,7 @@ int uploadCodingTables(const int* scan4, const int* scan8, const int* scan16, co
   for (int k = 0; k < 3; k++)
     for (int i = 0; i < (16 << (2 * k)); i++) {
       const int band = bandOf(i);
-      s[k][i] = (uint32_t)scans[k][i] | ((uint32_t)(band * kNumPrevClass * 64) << 8);
+      s[k][i] = (uint32_t)scans[k][i] | (uint32_t)band * dev::kGroupBytes << 8;
       pos[k][i] = (uint8_t)scans[k][i];
     }
   if (cudaMemcpyToSymbol(dev::cScanRow, s, sizeof(s)) != cudaSuccess) return kErrDevice;
