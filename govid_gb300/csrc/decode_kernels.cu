@@ -663,9 +663,8 @@ __device__ __forceinline__ bool symbolChain(const FrameDesc* fp, int tile, const
 }
 
 // Entropy jobs: up to kEntropyWarps tiles of one frame per job, one warp per
-// tile, sharing the frame's symbol tables.  A tile runs the symbol chain
-// when its frame has a symbol log (the full chain when it leaves the tile),
-// else the full chain.  With a queue counter the grid is
+// tile, sharing the frame's symbol tables.  A tile runs the symbol chain, and
+// the full chain when that leaves it.  With a queue counter the grid is
 // persistent: each CTA takes jobs (longest first, as listed) until none are
 // left, so a round with more jobs than resident CTAs has no second-wave
 // tail; without one, CTA b runs job b.
@@ -685,16 +684,13 @@ __global__ void __launch_bounds__(32 * kEntropyWarps, 2) kEntropy(const FrameDes
     buildTables(sT, *fp->tables, threadIdx.x, blockDim.x);
     if (warp < job.z) {
       const int tile = job.y + warp;
+      const TileRange tr = fp->tiles[tile];
+      const int mbs = (tr.mbX1 - tr.mbX0) * (tr.mbY1 - tr.mbY0);
+      for (int k = lane; k < mbs; k += 32) fp->symOff[tr.mbBase + k] = kSkipOffset;
+      __syncwarp();
       bool done = false;
-      if (fp->symOff) {
-        const TileRange tr = fp->tiles[tile];
-        const int mbs = (tr.mbX1 - tr.mbX0) * (tr.mbY1 - tr.mbY0);
-        for (int k = lane; k < mbs; k += 32) fp->symOff[tr.mbBase + k] = kSkipOffset;
-        __syncwarp();
-        if (lane == 0) done = symbolChain(fp, tile, sT);
-        done = __shfl_sync(kFull, done ? 1 : 0, 0) != 0;
-      }
-      if (!done) fullChain(fp, tile, sT, lane);
+      if (lane == 0) done = symbolChain(fp, tile, sT);
+      if (!__shfl_sync(kFull, done ? 1 : 0, 0)) fullChain(fp, tile, sT, lane);
     }
     if (!next) return;
     __syncthreads();  // every warp is done with sT and sJob before the next job

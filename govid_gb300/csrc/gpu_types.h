@@ -103,9 +103,8 @@ struct FrameDesc {
   int32_t prevKey;
   int32_t pad2;
   uint8_t* dep;
-  // Symbol path of the entropy stage (null: every tile takes the full chain):
-  // per macroblock the entries of its log (at mbBase + raster index within the
-  // tile).
+  // Per macroblock the entries of its symbol log (at mbBase + raster index
+  // within the tile).
   uint32_t* symOff;
 };
 

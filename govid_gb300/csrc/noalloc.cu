@@ -55,7 +55,8 @@ constexpr size_t kOffCoef = a256(kOffRec + (size_t)kNAMaxMBs * sizeof(MBRec));
 constexpr size_t kOffMV = a256(kOffCoef + (size_t)kNAMaxMBs * kCoefPerMB * sizeof(uint32_t));
 constexpr size_t kOffLV = a256(kOffMV + (size_t)kNAMaxMBs * 2 * sizeof(int16_t));
 constexpr size_t kOffIntra = a256(kOffLV + (size_t)kNAMaxMBs * sizeof(int16_t));
-constexpr size_t kOffTS = a256(kOffIntra + 2 * (size_t)kNAMaxMBs * sizeof(uint32_t));
+constexpr size_t kOffSym = kOffIntra + (size_t)kNAMaxMBs * sizeof(uint32_t);
+constexpr size_t kOffTS = a256(kOffSym + (size_t)kNAMaxMBs * sizeof(uint32_t));
 constexpr size_t kOffPkt = a256(kOffTS + (size_t)kNAMaxMBs * sizeof(TileStat));
 constexpr size_t kNABytes = a256(kOffPkt + kNAMaxPacket);
 // The header's figure is part of the interface; the layout fits it.
@@ -118,6 +119,7 @@ void fillDesc(FrameDesc& fd, uint8_t* d, int which, const Geometry& g, const Pay
   fd.mvgrid = reinterpret_cast<int16_t*>(d + kOffMV);
   fd.lvgrid = reinterpret_cast<int16_t*>(d + kOffLV);
   fd.intraList = reinterpret_cast<uint32_t*>(d + kOffIntra);
+  fd.symOff = reinterpret_cast<uint32_t*>(d + kOffSym);
   fd.tileStat = reinterpret_cast<TileStat*>(d + kOffTS);
   fd.status = reinterpret_cast<int32_t*>(d + kOffStatus) + which;
   fd.gate = nullptr;
@@ -222,21 +224,22 @@ extern "C" int ebivgpu_decode_key_noalloc(const uint8_t* pkt, size_t n, uint8_t*
   const int4* de = reinterpret_cast<const int4*>(d + kOffEJobs);
   const int nt0 = (int)plan[0].tiles.size();
   auto groups = [](int nt) { return (nt + kEntropyTilesPerJob - 1) / kEntropyTilesPerJob; };
-  int maxTile = 0, maxKeys = 0;
-  for (const TileRange& t : plan[0].tiles) {
-    const int w = t.mbX1 - t.mbX0, h = t.mbY1 - t.mbY0;
-    maxTile = std::max(maxTile, w * h);
-    maxKeys = std::max(maxKeys, 4 * (w - 1) + 11 * (h - 1) + 1);
-  }
+  int maxTile[2] = {0, 0}, maxKeys = 0;
+  for (int k = 0; k < payloads; k++)
+    for (const TileRange& t : plan[k].tiles) {
+      const int w = t.mbX1 - t.mbX0, h = t.mbY1 - t.mbY0;
+      maxTile[k] = std::max(maxTile[k], w * h);
+      if (k == 0) maxKeys = std::max(maxKeys, 4 * (w - 1) + 11 * (h - 1) + 1);
+    }
   // Each launch is checked where it is made.
-  launchEntropy(dd, de, groups(nt0), nullptr, (int)mbs, s);
+  launchEntropy(dd, de, groups(nt0), nullptr, maxTile[0], s);
   if (cudaGetLastError() != cudaSuccess) return kErrDevice;
   launchInter(dd, 1, (int)mbs, 0, s);  // the intra macroblocks' residuals
   if (cudaGetLastError() != cudaSuccess) return kErrDevice;
-  launchIntra(dd, dj, nt0, maxTile, maxKeys, 0, s);
+  launchIntra(dd, dj, nt0, maxTile[0], maxKeys, 0, s);
   if (cudaGetLastError() != cudaSuccess) return kErrDevice;
   if (withOv) {  // after the key's reconstruction, which reads the records it overwrites
-    launchEntropy(dd, de + kNAMaxEJobs, groups((int)plan[1].tiles.size()), nullptr, (int)mbs, s);
+    launchEntropy(dd, de + kNAMaxEJobs, groups((int)plan[1].tiles.size()), nullptr, maxTile[1], s);
     if (cudaGetLastError() != cudaSuccess) return kErrDevice;
   }
   if (cudaMemcpyAsync(status, d + kOffStatus, sizeof(status), cudaMemcpyDeviceToHost, s) != cudaSuccess ||

@@ -1,0 +1,54 @@
+"""What the entropy stage costs where it is not in its ordinary course, against that course on the same tile."""
+import ctypes as C
+import statistics
+import time
+
+import numpy as np
+import pytest
+
+import ebiv_oracle
+from govid_gb300 import _native, ebiv
+
+pytestmark = pytest.mark.gpu
+
+W, H = 640, 368
+
+
+def _key(seed=3, most=60):
+    """A key frame of one tile, about 100 symbols a macroblock: its chain is nearly all of its decode's time."""
+    rng = np.random.default_rng(seed)
+    mbs = (W // 16) * (H // 16)
+    levels = np.zeros((mbs, 384), np.int32)
+    at = rng.integers(0, 384, (mbs, most))
+    levels[np.arange(mbs)[:, None], at] = rng.integers(-3, 4, (mbs, most))
+    return ebiv.encode_key_from_levels(W, H, 20, 0, levels)
+
+
+def _ms(f, n=7):
+    f()
+    took = []
+    for _ in range(n):
+        t0 = time.perf_counter()
+        f()
+        took.append(1000 * (time.perf_counter() - t0))
+    return statistics.median(took)
+
+
+def test_key_frames_without_allocation_take_the_time_of_the_codec(gpu_required):
+    # Both are synchronous calls and wait for one chain; the codec copies the frame to the host as well.  Decoded by
+    # the full chain a key frame takes 2.5 times the chain's time and more.
+    import torch
+
+    pkt = _key()
+    y = torch.empty(W * H, dtype=torch.uint8, device="cuda")
+    cb, cr = (torch.empty(W * H // 4, dtype=torch.uint8, device="cuda") for _ in range(2))
+    w, h = C.c_int32(), C.c_int32()
+
+    def noalloc():
+        assert _native.lib().ebivgpu_decode_key_noalloc(pkt, len(pkt), y.data_ptr(), W, W * H, cb.data_ptr(),
+                                                        cr.data_ptr(), W // 2, W * H // 4, None, C.byref(w), C.byref(h)) == 0
+
+    codec = ebiv.Codec()
+    a, b = _ms(noalloc), _ms(lambda: codec.decode(pkt))
+    assert a < 1.5 * b, f"no allocation {a:.2f} ms, codec {b:.2f} ms"
+    assert b"".join(p.cpu().numpy().tobytes() for p in (y, cb, cr)) == ebiv_oracle.decode_all([pkt])[0][1]
