@@ -165,31 +165,20 @@ struct WarpChain {
     return (int)((e.w >> kLogShift) & 15u);
   }
   __device__ __forceinline__ int sym(int ctx) { return symAt(rowOf(ctx)); }
-  // Initialises the four states from the end of the tile's bytes
-  // (ransDecoder.reset, ebiv/rans.go:236-250); false when the stream is too short.
-  __device__ __forceinline__ bool reset(const uint8_t* b, uint32_t len, const EntropyTables* tables) {
+  // Takes up a tile's decoding (b: its bytes).
+  __device__ __forceinline__ void set(const uint8_t* b, const ChainState& s, const EntropyTables* tables) {
     buf = b;
-    pos = (int32_t)len;
     err = 0;
     t = tables;
-    if (len < (uint32_t)(kStates * 4)) {
-      err = kErrCorrupt;
-      return false;
-    }
-    uint32_t st[4];
-#pragma unroll
-    for (int i = kStates - 1; i >= 0; i--) {
-      st[i] = byteAt(pos - 1) << 24 | byteAt(pos - 2) << 16 | byteAt(pos - 3) << 8 | byteAt(pos - 4);
-      pos -= 4;
-    }
-    x0 = st[0];
-    x1 = st[1];
-    x2 = st[2];
-    x3 = st[3];
+    x0 = s.x0;
+    x1 = s.x1;
+    x2 = s.x2;
+    x3 = s.x3;
+    pos = s.pos;
     b1 = byteAt(pos - 1);
     b2 = byteAt(pos - 2);
-    return true;
   }
+  __device__ __forceinline__ ChainState state() const { return ChainState{x0, x1, x2, x3, pos}; }
 };
 
 // getRawBits / getClassValue / getMVComponent — ebiv/mv.go:75-128.
@@ -599,72 +588,99 @@ __device__ __forceinline__ uint32_t* coefRegion(const FrameDesc* fp, int idx) {
   return fp->coef + (size_t)idx * kCoefPerMB;
 }
 
-// The full chain of a tile, by one warp (the frame's tables are in sT): the
-// rANS symbols drive the macroblock grammar, and every macroblock reached
-// gets its record (inter vectors as deltas), its coefficient regions and,
-// when it is intra and written, an entry in the tile's intra list (raster
-// order).  Returns the macroblocks reached (all of them unless the chain
-// stopped at an error).
-__device__ __noinline__ int fullChain(const FrameDesc* fp, int tile, const EntropyTables& sT, int lane) {
-  const int mbCols = fp->mbCols;
-  const int inter = fp->inter;
-  MBRec* const recs = fp->mbrec;
+// The full chain, by one warp (the frame's tables are in sT): the rANS symbols
+// drive the macroblock grammar from macroblock `from` of the tile on, where
+// the decoder stands at *st, up to `to`, and every macroblock reached gets its
+// record (inter vectors as deltas), its coefficient regions and its flags.
+// Returns the macroblocks reached, with *st behind the last one, or with
+// st->pos -1 after an error, the macroblock where it came counted.
+__device__ __noinline__ int fullChain(const FrameDesc* fp, int tile, const EntropyTables& sT, int lane, ChainState* st,
+                                      int from, int to) {
   const TileRange tr = fp->tiles[tile];
-  uint32_t* const intraList = fp->intraList + tr.mbBase;
-  const int x0 = tr.mbX0, x1 = tr.mbX1, y0 = tr.mbY0, y1 = tr.mbY1;
-  const int tw = x1 - x0, total = tw * (y1 - y0);
+  const int tw = tr.mbX1 - tr.mbX0;
+  uint8_t* const flags = reinterpret_cast<uint8_t*>(fp->lvgrid) + tr.mbBase;
   WarpChain d;
-  d.reset(fp->pkt + tr.offset, tr.length, &sT);
-  int done = 0, intraCount = 0;
-  for (int mby = y0; mby < y1 && !d.err; mby++) {
-    for (int mbx = x0; mbx < x1; mbx++) {
-      const int idx = mby * mbCols + mbx;
-      if (decodeMB(d, inter, recs + idx, coefRegion(fp, idx), lane)) {
-        if (lane == 0) intraList[intraCount] = (uint32_t)idx;
-        intraCount++;
-      }
-      done++;
-      if (d.err) break;
+  d.set(fp->pkt + tr.offset, *st, &sT);
+  int k = from;
+  while (k < to && !d.err) {
+    const int idx = (tr.mbY0 + k / tw) * fp->mbCols + tr.mbX0 + k % tw;
+    const int f = decodeMB(d, fp->inter, fp->mbrec + idx, coefRegion(fp, idx), lane);
+    if (lane == 0) {
+      flags[k] = (uint8_t)f;
+      fp->symOff[tr.mbBase + k] = kDecodedOffset;
     }
+    k++;
   }
-  // Macroblocks the tile never reached are left untouched by reconstruction.
-  for (int k = done + lane; k < total; k += 32) {
-    MBRec* r = recs + (size_t)(y0 + k / tw) * mbCols + x0 + k % tw;
-    r->mode = kRecNone;
-    r->wmask = 0;
-  }
-  if (lane == 0) {
-    TileStat ts;
-    ts.err = d.err;
-    ts.intraCount = intraCount;
-    ts.done = done;
-    ts.fullChain = 1;
-    fp->tileStat[tile] = ts;
-    if (d.err) atomicExch(fp->status, kErrCorrupt);
-  }
-  return done;
+  *st = d.state();
+  if (d.err) st->pos = -1;
+  return k;
 }
 
-// The symbol chain of a tile, by one thread (Chain); false when it leaves the
-// tile to the full chain.
-__device__ __forceinline__ bool symbolChain(const FrameDesc* fp, int tile, const EntropyTables& sT) {
+// The symbol chain of a tile from macroblock `from` on, by one thread (Chain).
+// Returns the macroblocks decoded, with *st behind the last one, and in *next
+// the first one behind those that it leaves to the full chain.  Where it
+// failed, the decoder's state is not known; a second run up to the last
+// macroblock that is surely complete finds it.
+__device__ __forceinline__ int symbolChain(const FrameDesc* fp, const TileRange& tr, const EntropyTables& sT,
+                                           ChainState* st, int from, int* next) {
+  const int tw = tr.mbX1 - tr.mbX0;
+  uint16_t* const log = reinterpret_cast<uint16_t*>(coefRegion(fp, tr.mbY0 * fp->mbCols + tr.mbX0));
+  int upTo = tw * (tr.mbY1 - tr.mbY0);
+  Chain d;
+#pragma unroll 1
+  while (!d.run(fp->pkt + tr.offset, *st, sT, fp->inter, from, upTo, log, kLogEntries, fp->symOff + tr.mbBase, tw,
+                fp->mbCols)) {
+    *next = d.mb + 1;
+    upTo = d.reached(from);
+    if (upTo == from) return from;
+  }
+  *st = d.state();
+  return upTo;
+}
+
+// A tile, by one warp: the symbol chain as far as it goes, the full chain for
+// the macroblocks that it leaves (one with no room for its log; one where a
+// symbol fails, which ends the tile), and so on.  A tile with an error takes
+// two passes of the symbol chain up to there, which are quicker together than
+// the full chain's one.
+__device__ __forceinline__ void decodeTile(const FrameDesc* fp, int tile, const EntropyTables& sT, int lane) {
   const TileRange tr = fp->tiles[tile];
   const int tw = tr.mbX1 - tr.mbX0, total = tw * (tr.mbY1 - tr.mbY0);
-  uint16_t* const log = reinterpret_cast<uint16_t*>(coefRegion(fp, tr.mbY0 * fp->mbCols + tr.mbX0));
-  Chain d;
-  if (!d.run(fp->pkt + tr.offset, tr.length, sT, fp->inter, total, log, kLogEntries, fp->symOff + tr.mbBase, tw,
-             fp->mbCols))
-    return false;
-  TileStat* ts = fp->tileStat + tile;
-  ts->err = 0;
-  ts->done = total;
-  ts->fullChain = 0;
-  return true;
+  uint32_t* const entries = fp->symOff + tr.mbBase;
+  for (int k = lane; k < total; k += 32) entries[k] = kSkipOffset;
+  __syncwarp();
+  ChainState st = {0u, 0u, 0u, 0u, -1};
+  if (tr.length >= (uint32_t)(kStates * 4)) st = initialState(fp->pkt + tr.offset, tr.length);
+  int done = 0;
+  while (st.pos >= 0 && done < total) {
+    int next = 0;
+    if (lane == 0) done = symbolChain(fp, tr, sT, &st, done, &next);
+    done = __shfl_sync(kFull, done, 0);
+    if (done == total) break;
+    next = __shfl_sync(kFull, next, 0);
+    st.x0 = __shfl_sync(kFull, st.x0, 0);
+    st.x1 = __shfl_sync(kFull, st.x1, 0);
+    st.x2 = __shfl_sync(kFull, st.x2, 0);
+    st.x3 = __shfl_sync(kFull, st.x3, 0);
+    st.pos = __shfl_sync(kFull, st.pos, 0);
+    done = fullChain(fp, tile, sT, lane, &st, done, next);
+  }
+  const bool err = st.pos < 0;
+  // Macroblocks the tile never reached are left untouched by reconstruction.
+  for (int k = done + lane; k < total; k += 32) {
+    MBRec* r = fp->mbrec + (size_t)(tr.mbY0 + k / tw) * fp->mbCols + tr.mbX0 + k % tw;
+    r->mode = kRecNone;
+    r->wmask = 0;
+    entries[k] = kDecodedOffset;
+  }
+  if (lane == 0) {
+    fp->tileStat[tile] = TileStat{err ? kErrCorrupt : 0, 0, done, 0};
+    if (err) atomicExch(fp->status, kErrCorrupt);
+  }
 }
 
 // Entropy jobs: up to kEntropyWarps tiles of one frame per job, one warp per
-// tile, sharing the frame's symbol tables.  A tile runs the symbol chain, and
-// the full chain when that leaves it.  With a queue counter the grid is
+// tile, sharing the frame's symbol tables.  With a queue counter the grid is
 // persistent: each CTA takes jobs (longest first, as listed) until none are
 // left, so a round with more jobs than resident CTAs has no second-wave
 // tail; without one, CTA b runs job b.
@@ -682,22 +698,13 @@ __global__ void __launch_bounds__(32 * kEntropyWarps, 2) kEntropy(const FrameDes
     const int4 job = jobs[jb];
     const FrameDesc* fp = frames + job.x;
     buildTables(sT, *fp->tables, threadIdx.x, blockDim.x);
-    if (warp < job.z) {
-      const int tile = job.y + warp;
-      const TileRange tr = fp->tiles[tile];
-      const int mbs = (tr.mbX1 - tr.mbX0) * (tr.mbY1 - tr.mbY0);
-      for (int k = lane; k < mbs; k += 32) fp->symOff[tr.mbBase + k] = kSkipOffset;
-      __syncwarp();
-      bool done = false;
-      if (lane == 0) done = symbolChain(fp, tile, sT);
-      if (!__shfl_sync(kFull, done ? 1 : 0, 0)) fullChain(fp, tile, sT, lane);
-    }
+    if (warp < job.z) decodeTile(fp, job.y + warp, sT, lane);
     if (!next) return;
     __syncthreads();  // every warp is done with sT and sJob before the next job
   }
 }
 
-// Rebuilds the records of the symbol-path tiles from their logs, one warp
+// Rebuilds the records of the logged macroblocks, one warp
 // per macroblock over every macroblock of the launch's tiles (grid.x: job *
 // kEntropyTilesPerJob + tile within the job; grid.y * kParseWarps: the
 // macroblock's raster index within its tile).  A skip macroblock's record is
@@ -830,7 +837,6 @@ __global__ void __launch_bounds__(32 * kParseWarps) kParseMB(const FrameDesc* fr
   if (tj >= job.z) return;
   const FrameDesc* fp = frames + job.x;
   const int tile = job.y + tj;
-  if (fp->tileStat[tile].fullChain) return;
   const TileRange tr = fp->tiles[tile];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tw = tr.mbX1 - tr.mbX0, total = tw * (tr.mbY1 - tr.mbY0);
@@ -840,6 +846,7 @@ __global__ void __launch_bounds__(32 * kParseWarps) kParseMB(const FrameDesc* fr
   uint4* const words = reinterpret_cast<uint4*>(fp->mbrec + idx);
   uint8_t* const flags = reinterpret_cast<uint8_t*>(fp->lvgrid) + tr.mbBase;
   const uint32_t entries = fp->symOff[tr.mbBase + k];
+  if (entries == kDecodedOffset) return;
   if (entries == kSkipOffset) {
     if (lane < 3) words[lane] = make_uint4(lane ? 0u : (uint32_t)kRecSkip, 0u, 0u, lane == 2 ? kWriteAll : 0u);
     if (lane == 0) flags[k] = 0;
@@ -996,8 +1003,7 @@ __device__ void predictVectorsShared(const FrameDesc* fp, const TileRange& tr, i
 
 // After kParseMB: per tile (one CTA per tile of a job) the written intra
 // macroblocks listed in raster order, and (inter frames) the tile's vector
-// wavefront.  Tiles the full chain decoded have their intra list already;
-// only the wavefront runs for them.
+// wavefront.
 constexpr int kFlagsPerThread = 8;
 __global__ void __launch_bounds__(kFinishThreads) kTileFinish(const FrameDesc* frames, const int4* jobs, int njobs) {
   __shared__ union {
@@ -1016,37 +1022,35 @@ __global__ void __launch_bounds__(kFinishThreads) kTileFinish(const FrameDesc* f
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int mbCols = fp->mbCols, tw = tr.mbX1 - tr.mbX0;
   const int done = st.done;
-  if (!st.fullChain) {
-    // Each thread counts the flags of eight macroblocks in a row, a warp and
-    // then the CTA add the counts up, and each thread lists its own.
-    const uint8_t* const flags = reinterpret_cast<const uint8_t*>(fp->lvgrid) + tr.mbBase;
-    int base = 0;
-    for (int k0 = 0; k0 < done; k0 += kFinishThreads * kFlagsPerThread) {
-      const int k = k0 + tid * kFlagsPerThread;
-      uint32_t set = 0;
+  // Each thread counts the flags of eight macroblocks in a row, a warp and
+  // then the CTA add the counts up, and each thread lists its own.
+  const uint8_t* const flags = reinterpret_cast<const uint8_t*>(fp->lvgrid) + tr.mbBase;
+  int base = 0;
+  for (int k0 = 0; k0 < done; k0 += kFinishThreads * kFlagsPerThread) {
+    const int k = k0 + tid * kFlagsPerThread;
+    uint32_t set = 0;
 #pragma unroll
-      for (int j = 0; j < kFlagsPerThread; j++)
-        if (k + j < done && flags[k + j] != 0) set |= 1u << j;
-      int upTo = __popc(set);
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(kFull, upTo, o);
-        if (lane >= o) upTo += v;
-      }
-      if (lane == 31) sWarp[warp] = upTo;
-      __syncthreads();
-      int at = base + upTo - __popc(set);
-      for (int w = 0; w < kFinishThreads / 32; w++) {
-        if (w < warp) at += sWarp[w];
-        base += sWarp[w];
-      }
-      for (; set; set &= set - 1) {
-        const int m = k + __ffs(set) - 1;
-        fp->intraList[tr.mbBase + at++] = (uint32_t)((tr.mbY0 + m / tw) * mbCols + tr.mbX0 + m % tw);
-      }
-      __syncthreads();
+    for (int j = 0; j < kFlagsPerThread; j++)
+      if (k + j < done && flags[k + j] != 0) set |= 1u << j;
+    int upTo = __popc(set);
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(kFull, upTo, o);
+      if (lane >= o) upTo += v;
     }
-    if (tid == 0) fp->tileStat[tile].intraCount = base;
+    if (lane == 31) sWarp[warp] = upTo;
+    __syncthreads();
+    int at = base + upTo - __popc(set);
+    for (int w = 0; w < kFinishThreads / 32; w++) {
+      if (w < warp) at += sWarp[w];
+      base += sWarp[w];
+    }
+    for (; set; set &= set - 1) {
+      const int m = k + __ffs(set) - 1;
+      fp->intraList[tr.mbBase + at++] = (uint32_t)((tr.mbY0 + m / tw) * mbCols + tr.mbX0 + m % tw);
+    }
+    __syncthreads();
   }
+  if (tid == 0) fp->tileStat[tile].intraCount = base;
   if (!fp->inter) return;
   if (tw <= kRowMax) predictVectorsShared(fp, tr, done, sV.vectors, tid);
   else if (warp == 0) predictVectors(fp, tile, done, sV.rows, lane);

@@ -60,7 +60,7 @@ struct TileStat {
   int32_t err;         // 0 or an ebiv status
   int32_t intraCount;  // intra macroblocks reconstructed in this tile
   int32_t done;        // macroblocks the tile's chain reached (raster order)
-  int32_t fullChain;   // 1: the full chain decoded the tile (its records and intra list are complete)
+  int32_t pad;
 };
 
 // Intra list entries hold the frame macroblock index in bits 0-17.

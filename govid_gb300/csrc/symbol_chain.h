@@ -105,6 +105,7 @@ constexpr uint32_t kLogToken = 0, kLogSign = 1u << 6, kLogMode = 2u << 6, kLogVa
 constexpr int kLogShift = 8;
 constexpr uint32_t kLogNonzero = 4;               // token flag, where Chain::far looks
 constexpr uint32_t kSkipOffset = 0xFFFFFFFFu;     // a skip macroblock: it has no log
+constexpr uint32_t kDecodedOffset = 0xFFFFFFFEu;  // one that the full chain has decoded, or that is not reached
 // The entries of a macroblock's header (mode, reference, partition, eight
 // vector components, pattern, transform size), the most that n blocks with
 // `coefs` coefficients take without escapes (a token and a sign for each
@@ -163,6 +164,26 @@ EBIV_DEV uint4 blockEntry(int kind) {
                     (mode ? row : row + kGroupBytes) + (2048 - edge) * kECount + (rest ? kERest : 0u),
                     mode ? (1u | 1u << 2 | 1u << 8) << 12 : (1u << 1 | 1u << 7 | 1u << 19) << 12,
                     rest ? (2048 - (total - 19)) * kECount : 0u);
+}
+
+// Where a tile's rANS decoder stands between two symbols: its states in use
+// order and the stream bytes not taken yet (it reads them backwards).
+struct ChainState {
+  uint32_t x0, x1, x2, x3;
+  int32_t pos;
+};
+// The state at a tile's start, from the end of its len >= 16 bytes
+// (ransDecoder.reset, ebiv/rans.go:236-250).
+EBIV_DEV ChainState initialState(const uint8_t* buf, uint32_t len) {
+  uint32_t st[kStates];
+  int pos = (int)len;
+#pragma unroll
+  for (int i = kStates - 1; i >= 0; i--) {
+    st[i] = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) st[i] = st[i] << 8 | (uint32_t)__ldg(buf + --pos);
+  }
+  return ChainState{st[0], st[1], st[2], st[3], pos};
 }
 
 // A tile's chain, run by one thread.
@@ -627,27 +648,17 @@ struct Chain {
     return mode;
   }
 
-  // Initialises the four states from the end of the tile's bytes
-  // (ransDecoder.reset, ebiv/rans.go:236-250); false when the stream is too
-  // short, or when a state is below kLower or at 2^31 and above, as no encoder
-  // leaves it (a symbol of one in between takes at most two bytes and leaves
-  // one).  The bytes down to the first aligned word are read one by one, so no
-  // load reaches past the tile.
-  EBIV_DEV bool reset(const uint8_t* buf, uint32_t len, const EntropyTables* tables) {
+  // Takes up a tile's decoding (buf: its bytes); false when a state is below
+  // kLower or at 2^31 and above, as no encoder leaves it (a symbol of one in
+  // between takes at most two bytes and leaves one).  The bytes down to the
+  // first aligned word are read one by one, so no load reaches past the tile.
+  EBIV_DEV bool set(const uint8_t* buf, const ChainState& s, const EntropyTables* tables) {
     t = tables;
-    if (len < (uint32_t)(kStates * 4)) return false;
-    int pos = (int)len;
-    uint32_t st[kStates];
-#pragma unroll
-    for (int i = kStates - 1; i >= 0; i--) {
-      st[i] = 0;
-#pragma unroll
-      for (int k = 0; k < 4; k++) st[i] = st[i] << 8 | (uint32_t)__ldg(buf + --pos);
-    }
-    x0 = st[0];
-    x1 = st[1];
-    x2 = st[2];
-    x3 = st[3];
+    x0 = s.x0;
+    x1 = s.x1;
+    x2 = s.x2;
+    x3 = s.x3;
+    int pos = s.pos;
     if (min(min(x0, x1), min(x2, x3)) < kLower || ((x0 | x1 | x2 | x3) >> 31) != 0) return false;
     rem = 8 * pos;
     const int head = min(pos, (int)((uintptr_t)(buf + pos) & 3));  // bytes above the last aligned word
@@ -661,15 +672,21 @@ struct Chain {
     return true;
   }
 
-  // The chain of a tile: len bytes at buf, total macroblocks.  Its log goes
-  // into tileLog, which has `entries` entries, or with a tile width as many for
-  // each macroblock of a frame `stride` macroblocks wide, of which tileLog
-  // holds the tile's first.  offsets (kSkipOffset everywhere before) gets the
-  // first entry of each macroblock that is not skip, with a tile width the
-  // number of its entries.  False when the tile is left to the full chain: a
-  // symbol failed, or there was no room for the most entries that could
-  // follow.
+  // The chain of a whole tile: len bytes at buf, its log into tileLog.
   EBIV_DEV bool run(const uint8_t* buf, uint32_t len, const EntropyTables& tables, int inter, int total,
+                    uint16_t* tileLog, int entries, uint32_t* offsets, int tileWidth = 0, int stride = 0) {
+    return len >= (uint32_t)(kStates * 4) &&
+           run(buf, initialState(buf, len), tables, inter, 0, total, tileLog, entries, offsets, tileWidth, stride);
+  }
+  // The chain of a tile's macroblocks from `from` on, where its decoder stands
+  // at s, up to macroblock `total`.  Its log goes into tileLog, which has
+  // `entries` entries, or with a tile width as many for each macroblock of a
+  // frame `stride` macroblocks wide, of which tileLog holds the tile's first.
+  // offsets (kSkipOffset everywhere before) gets the first entry of each
+  // macroblock that is not skip, with a tile width the number of its entries.
+  // False when macroblocks from reached() on are left to the full chain: a
+  // symbol failed, or there was no room for the most entries that could follow.
+  EBIV_DEV bool run(const uint8_t* buf, const ChainState& s, const EntropyTables& tables, int inter, int from, int total,
                     uint16_t* tileLog, int entries, uint32_t* offsets, int tileWidth = 0, int stride = 0) {
     log = lp = tileLog;
     end = log + entries;
@@ -679,9 +696,10 @@ struct Chain {
     mbOff = offsets;
     stop = total;
     intraOnly = !inter;
-    if (!reset(buf, len, &tables)) return false;
+    mb = from;
+    if (!set(buf, s, &tables)) return false;
 #pragma unroll 1
-    for (mb = 0; mb < stop; mb++) {
+    for (; mb < stop; mb++) {
       uint32_t mode = mbIntra;
       if (inter) {
         mode = skips(mb, &mb);
@@ -718,6 +736,13 @@ struct Chain {
     }
     return stop == total;
   }
+  // After run(): where the decoder stands behind the last macroblock.
+  EBIV_DEV ChainState state() const { return ChainState{x0, x1, x2, x3, rem >> 3}; }
+  // After a run() from macroblock `from` on that failed in macroblock mb: the
+  // macroblocks surely complete.  In a frame of intra macroblocks only, the
+  // failing symbol may be up to three before the one where that was noticed,
+  // at the end of the macroblock before.
+  EBIV_DEV int reached(int from) const { return intraOnly && mb > from ? mb - 1 : mb; }
 };
 
 }  // namespace dev

@@ -1,7 +1,8 @@
 // The symbol chain with the log as the entropy kernel has it: each macroblock's
 // entries in a room of their own inside the frame's coefficient regions
-// (kSymPerMB bytes), for every tile of every packet the planner accepts,
-// against the plain decoder of chain_test.cpp.  Rooms of other tiles and of
+// (kSymPerMB bytes), for every tile of every packet the planner accepts, and
+// taken up again behind macroblocks that it leaves, against the plain decoder
+// of chain_test.cpp.  Rooms of other tiles and of
 // skip macroblocks, and a room behind its entries, stay as they were; the
 // frame's regions are allocated at their exact size.
 //
@@ -10,7 +11,11 @@
 #include "chain_test.cpp"
 #undef main
 
+#include <algorithm>
+
 namespace {
+
+using dev::ChainState;
 
 constexpr int kRoom = kSymPerMB / 2;
 constexpr uint16_t kUntouched = 0xBEEF;
@@ -27,57 +32,103 @@ struct Rooms {
   uint16_t* at(int x, int y) { return log.get() + ((size_t)y * cols + x) * kRoom; }
 };
 
-long compared = 0, small = 0, macroblocks = 0, dense = 0;
+long compared = 0, small = 0, logged = 0, dense = 0, stopped = 0, resumed = 0;
 
+ChainState stateOf(const Plain& p) {
+  auto x = [&](int i) { return p.x[(p.at + i) & 3]; };
+  return ChainState{x(0), x(1), x(2), x(3), p.pos};
+}
+bool same(const ChainState& a, const ChainState& b) {
+  return a.x0 == b.x0 && a.x1 == b.x1 && a.x2 == b.x2 && a.x3 == b.x3 && a.pos == b.pos;
+}
+
+// As the kernel decodes a tile: the chain as far as it goes, the plain decoder
+// for the macroblocks that it leaves, the chain again behind them.
 const char* sameRooms(const PayloadPlan& p, const TileRange& r, const uint8_t* pkt, bool inter,
                       const dev::EntropyTables& tables, const Geometry& geo) {
   const int tw = r.mbX1 - r.mbX0, total = tw * (r.mbY1 - r.mbY0);
-  Plain want(p.tables, pkt + r.offset, (int)r.length);
-  want.run(inter, total);
+  const uint8_t* const buf = pkt + r.offset;
+  Plain want(p.tables, buf, (int)r.length);
   tiles++;
+  if (want.err) {  // too short for the states: nothing runs
+    failing++;
+    return nullptr;
+  }
+  std::vector<ChainState> before;  // where the plain decoder stands before each macroblock
+  std::vector<size_t> at;
+  for (int k = 0; k < total && !want.err; k++) {
+    before.push_back(stateOf(want));
+    at.push_back(want.log.size());
+    want.run(inter, 1);
+  }
   failing += want.err;
-  int largest = 0, at = (int)want.log.size();
-  for (size_t k = want.off.size(); k-- > 0;)
-    if (want.off[k] != dev::kSkipOffset) {
-      largest = std::max(largest, at - (int)want.off[k]);
-      at = (int)want.off[k];
-    }
+  const int good = (int)before.size() - (want.err ? 1 : 0);  // macroblocks without an error
+  before.push_back(stateOf(want));
+  at.push_back(want.log.size());
+  int largest = 0;
+  for (int k = 0; k < good; k++) largest = std::max(largest, (int)(at[(size_t)k + 1] - at[(size_t)k]));
   Rooms rooms(geo.mbCols, geo.mbRows);
   std::vector<uint32_t> entries((size_t)total, dev::kSkipOffset);
-  dev::Chain d;
-  const bool whole = d.run(pkt + r.offset, r.length, tables, inter, total, rooms.at(r.mbX0, r.mbY0), kRoom,
-                           entries.data(), tw, geo.mbCols);
-  if (!whole) {
-    if (!want.err && !want.low && largest <= kAlwaysFits) return "left although it fits";
-    dense += !want.err && !want.low;
-  } else {
-    if (want.err) return "a failing tile decoded";
-    compared++;
-    small += total <= 6 && !want.log.empty();
+  std::vector<char> mine((size_t)total, 0);  // logged by the chain
+  ChainState st = before[0];
+  int done = 0;
+  long left = 0;
+  while (done < total) {
+    int upTo = total, next = 0;
+    dev::Chain d;
+    bool again = false;
+    while (!d.run(buf, st, tables, inter, done, upTo, rooms.at(r.mbX0, r.mbY0), kRoom, entries.data(), tw, geo.mbCols)) {
+      if (again) return "the second run failed";
+      next = d.mb + 1;
+      upTo = d.reached(done);
+      if (upTo < done || upTo >= next || next - upTo > 2) return "no progress";
+      if (upTo == done) break;
+      again = true;
+    }
+    if (upTo > good) return "decoded beyond an error";
+    if (upTo > done) {
+      if (!same(d.state(), before[(size_t)upTo])) return "another state behind the last macroblock";
+      std::fill(mine.begin() + done, mine.begin() + upTo, 1);
+    }
+    resumed += done > 0 && upTo > done;
+    done = upTo;
+    if (done == total) break;
+    left += next - done;
+    if (next > good) {  // the plain decoder meets the error there
+      if (!want.err) return "left behind the end";
+      stopped++;
+      break;
+    }
+    std::fill(entries.begin() + done, entries.begin() + next, dev::kDecodedOffset);
+    done = next;
+    st = before[(size_t)done];
   }
-  std::vector<uint32_t> next(want.off);
-  next.push_back((uint32_t)want.log.size());
-  for (size_t k = next.size() - 1; k-- > 0;)
-    if (next[k] == dev::kSkipOffset) next[k] = next[k + 1];  // where macroblock k's entries would begin
+  if (want.err && done > good) return "no error";
+  // Without an error only macroblocks with no room are left, and in a frame of intra macroblocks the one before.
+  if (!want.err && !want.low && left && largest <= kAlwaysFits) return "left although it fits";
+  dense += !want.err && !want.low && left;
+  compared++;
+  small += total <= 6 && std::count(mine.begin(), mine.end(), 1) == total && !want.log.empty();
   for (int y = 0; y < geo.mbRows; y++)
     for (int x = 0; x < geo.mbCols; x++) {
       const bool inside = x >= r.mbX0 && x < r.mbX1 && y >= r.mbY0 && y < r.mbY1;
-      const int k = inside ? (y - r.mbY0) * tw + x - r.mbX0 : 0;
+      const size_t k = inside ? (size_t)((y - r.mbY0) * tw + x - r.mbX0) : 0;
+      if (inside && !mine[k]) continue;
       const uint16_t* const room = rooms.at(x, y);
       int used = 0;
-      if (inside && whole) {
-        if ((want.off[(size_t)k] == dev::kSkipOffset) != (entries[(size_t)k] == dev::kSkipOffset)) return "skip differs";
-        if (want.off[(size_t)k] != dev::kSkipOffset) {
-          used = (int)entries[(size_t)k];
-          macroblocks++;
-          if (used != (int)(next[(size_t)k + 1] - want.off[(size_t)k])) return "number of entries differs";
-          if (std::memcmp(room, want.log.data() + want.off[(size_t)k], 2 * (size_t)used)) return "entries differ";
+      if (inside) {
+        const bool skip = want.off[k] == dev::kSkipOffset;
+        if (skip != (entries[k] == dev::kSkipOffset)) return "skip differs";
+        if (!skip) {
+          used = (int)entries[k];
+          logged++;
+          if (used != (int)(at[k + 1] - at[k])) return "number of entries differs";
+          if (std::memcmp(room, want.log.data() + at[k], 2 * (size_t)used)) return "entries differ";
           used = std::min(kRoom, used + 1);  // the next macroblock's transform size may stand there
         }
       }
-      if (!inside || whole)
-        for (int i = used; i < kRoom; i++)
-          if (room[i] != kUntouched) return "written outside the macroblock's entries";
+      for (int i = used; i < kRoom; i++)
+        if (room[i] != kUntouched) return "written outside the macroblock's entries";
     }
   return nullptr;
 }
@@ -131,7 +182,7 @@ int main(int argc, char** argv) {
         }
     }
   }
-  std::printf("tiles %ld failing %ld dense %ld compared %ld small %ld macroblocks %ld\n", tiles, failing, dense, compared,
-              small, macroblocks);
+  std::printf("tiles %ld failing %ld dense %ld compared %ld small %ld logged %ld stopped %ld resumed %ld\n", tiles, failing,
+              dense, compared, small, logged, stopped, resumed);
   return 0;
 }

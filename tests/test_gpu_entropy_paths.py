@@ -14,14 +14,25 @@ pytestmark = pytest.mark.gpu
 W, H = 640, 368
 
 
-def _key(seed=3, most=60):
-    """A key frame of one tile, about 100 symbols a macroblock: its chain is nearly all of its decode's time."""
+def _key(seed=3, most=60, full=()):
+    """A key frame of one tile, about 100 symbols a macroblock: its chain is nearly all of its decode's time.  The
+    macroblocks of `full` have all of their coefficients and many escapes, more than their log has room for."""
     rng = np.random.default_rng(seed)
     mbs = (W // 16) * (H // 16)
     levels = np.zeros((mbs, 384), np.int32)
     at = rng.integers(0, 384, (mbs, most))
     levels[np.arange(mbs)[:, None], at] = rng.integers(-3, 4, (mbs, most))
+    for m in full:
+        levels[m] = rng.choice([-1, 1], 384) * rng.integers(3, 9, 384)
     return ebiv.encode_key_from_levels(W, H, 20, 0, levels)
+
+
+def _status(codec, pkt):
+    try:
+        codec.decode(pkt)
+        return 0
+    except ebiv.EbivError as e:
+        return e.status
 
 
 def _ms(f, n=7):
@@ -52,3 +63,35 @@ def test_key_frames_without_allocation_take_the_time_of_the_codec(gpu_required):
     a, b = _ms(noalloc), _ms(lambda: codec.decode(pkt))
     assert a < 1.5 * b, f"no allocation {a:.2f} ms, codec {b:.2f} ms"
     assert b"".join(p.cpu().numpy().tobytes() for p in (y, cb, cr)) == ebiv_oracle.decode_all([pkt])[0][1]
+
+
+def _cut(pkt, n):
+    """The packet, of one tile, without the tile's first n bytes: read backwards, it fails near its end."""
+
+    def varint(v):
+        out = bytearray()
+        while v >= 128:
+            out.append(v & 127 | 128)
+            v >>= 7
+        return bytes(out) + bytes([v])
+
+    for at in range(6, 2000):
+        size = len(pkt) - at - 3
+        if pkt[at:at + 3] == varint(size):
+            return pkt[:at] + varint(size - n) + pkt[at + 3 + n:]
+    raise AssertionError("no tile")
+
+
+@pytest.mark.parametrize("what", ["error", "full"])
+def test_what_the_chain_leaves_costs_one_pass_more(gpu_required, what):
+    # A tile with an error and tiles with macroblocks that have no room for their log: a second pass of the symbol
+    # chain and these macroblocks by the full chain, which for a whole tile takes 2.5 passes by itself.
+    plain = _key()
+    pkt = _cut(plain, 100) if what == "error" else _key(full=(0, 17, 460, 461, 915))
+    codec = ebiv.Codec()
+    intact, other = _ms(lambda: codec.decode(plain)), _ms(lambda: _status(codec, pkt))
+    assert other < 2.5 * intact, f"intact {intact:.2f} ms, {what} {other:.2f} ms"
+    st, planes = ebiv_oracle.decode_all([pkt])[0]
+    assert _status(codec, pkt) == st == (ebiv.ErrCorrupt.status if what == "error" else 0)
+    if st == 0:
+        assert codec.decode(pkt).packed() == planes
