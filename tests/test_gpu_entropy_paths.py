@@ -9,6 +9,8 @@ import pytest
 import ebiv_oracle
 from govid_gb300 import _native, ebiv
 
+from helpers import encode_gen
+
 pytestmark = pytest.mark.gpu
 
 W, H = 640, 368
@@ -95,3 +97,21 @@ def test_what_the_chain_leaves_costs_one_pass_more(gpu_required, what):
     assert _status(codec, pkt) == st == (ebiv.ErrCorrupt.status if what == "error" else 0)
     if st == 0:
         assert codec.decode(pkt).packed() == planes
+
+
+@pytest.mark.parametrize("lookahead,depth", [(1, 0), (4, 0), (4, 2)])
+def test_more_jobs_than_ctas_of_several_frames(gpu_required, lookahead, depth):
+    # 1000 tiles a frame are 250 entropy jobs; four frames at once have 1000 for the 304 CTAs, which keep a frame's
+    # tables from one job to the next and change them with the frame.
+    cont, _, _ = encode_gen(640, 400, 8, ebiv.synth_pan, intra=14, gop=3, tiles=(40, 25), keep_recon=False)
+    pkts = [p.data for p in ebiv.Reader(cont).packets()]
+    want = ebiv_oracle.decode_all(pkts)
+    b = ebiv.Batch(lookahead=lookahead, pipeline=depth)
+    b.add_stream(pkts)
+    got = {}
+    for _ in range(len(pkts) + depth + 2):
+        for r in b.round():
+            got[r.frame_index] = (r.status, b.download(r, 640, 400))
+    for r in b.drain():
+        got[r.frame_index] = (r.status, b.download(r, 640, 400))
+    assert [got[i] for i in range(len(pkts))] == want
