@@ -46,10 +46,6 @@ __device__ uint8_t gScan[3][256];
 __device__ __align__(16) int32_t gDct[3][256];
 __constant__ int32_t cTaps[4][4] = {{0, 64, 0, 0}, {-6, 55, 18, -3}, {-8, 40, 40, -8}, {-3, 18, 55, -6}};
 
-__device__ __forceinline__ int tokenCtx(int plane, int txIdx, int band, int prevClass) {
-  return plane == kPlaneLuma ? ctxTokenBase + (txIdx * kNumBands + band) * kNumPrevClass + prevClass
-                             : ctxTokenBase + kLumaTokenCtx + band * kNumPrevClass + prevClass;
-}
 __device__ __forceinline__ int clampByteD(int32_t v) { return v < 0 ? 0 : (v > 255 ? 255 : v); }
 __device__ __forceinline__ int32_t wadd(int32_t a, int32_t b) { return (int32_t)((uint32_t)a + (uint32_t)b); }
 __device__ __forceinline__ int32_t wmul(int32_t a, int32_t b) { return (int32_t)((uint32_t)a * (uint32_t)b); }
@@ -61,11 +57,6 @@ __device__ __forceinline__ int16_t clampMV(int v) {
 // ---------------------------------------------------------------------------
 // Stage A: entropy decode
 // ---------------------------------------------------------------------------
-constexpr int kRowMax = 128;  // tiles at most this many macroblocks wide pass vector rows in shared memory
-struct WarpRows {
-  uint32_t mv[2][kRowMax];  // packed vectors of a pass's last row, by pass parity
-};
-
 // One warp per context in turn: lane s holds where symbol s starts and
 // writes its entry, then each lane finds two buckets' symbols among them.
 __device__ __forceinline__ void buildTables(EntropyTables& T, const DeviceTables& src, int tid, int nthreads) {
@@ -243,16 +234,6 @@ __device__ __forceinline__ int entropyBlock(WarpChain& d, uint32_t row, int sz, 
   return count;
 }
 
-__device__ __forceinline__ int16_t median3(int16_t a, int16_t b, int16_t c) {
-  if (a > b) {
-    const int16_t t = a;
-    a = b;
-    b = t;
-  }
-  if (b > c) b = c;
-  if (a > b) b = a;
-  return b;
-}
 __device__ __forceinline__ uint32_t packMV(int x, int y) { return (uint32_t)(uint16_t)x | ((uint32_t)(uint16_t)y << 16); }
 __device__ __forceinline__ int mvX(uint32_t v) { return (int16_t)(v & 0xFFFFu); }
 __device__ __forceinline__ int mvY(uint32_t v) { return (int16_t)(v >> 16); }
@@ -439,25 +420,24 @@ __device__ __forceinline__ uint32_t writeMask(const BlockPlan& p, int done) {
 // at step t, column t - 2k.  The left neighbour is the lane's own result of
 // the step before; the row above comes from lane k-1 by shuffle (its
 // results of the last three steps are columns x-1, x, x+1), and for lane 0
-// from the previous pass's last row (shared memory; the frame's vector grid
-// for tiles wider than kRowMax).  A skip macroblock takes the prediction;
-// an inter one adds its deltas (partition 0 to the prediction, zero for the
-// golden reference; later partitions to partition 0), clamped as the chain
-// would have.  Records past `done` are not touched.
-__device__ void predictVectors(const FrameDesc* fp, int tile, int done, WarpRows& rows, int lane) {
+// from the previous pass's last row, in the frame's vector grid.  A skip
+// macroblock takes the prediction; an inter one adds its deltas (partition 0 to
+// the prediction, zero for the golden reference; later partitions to partition
+// 0), clamped as the chain would have.  Records past `done` are not touched.
+// For tiles wider than kRowMax; predictVectorsShared has the others.
+__device__ void predictVectors(const FrameDesc* fp, int tile, int done, int lane) {
   const int mbCols = fp->mbCols;
   MBRec* const recs = fp->mbrec;
   uint32_t* const gmv = reinterpret_cast<uint32_t*>(fp->mvgrid);
   const TileRange tr = fp->tiles[tile];
   const int x0 = tr.mbX0, y0 = tr.mbY0, tw = tr.mbX1 - x0, th = tr.mbY1 - y0;
-  const bool wide = tw > kRowMax;
-  for (int p0 = 0, pass = 0; p0 < th; p0 += 32, pass++) {
+  for (int p0 = 0; p0 < th; p0 += 32) {
     const int ry = p0 + lane;
     const int nrows = min(32, th - p0);
     const int steps = tw + 2 * (nrows - 1);
     const bool lastRowOfPass = lane == 31 && p0 + 32 < th;
-    const uint32_t* upRow = wide ? gmv + (size_t)(y0 + p0 - 1) * mbCols + x0 : rows.mv[(pass + 1) & 1];
-    uint32_t* nextUp = wide ? gmv + (size_t)(y0 + p0 + 31) * mbCols + x0 : rows.mv[pass & 1];
+    const uint32_t* upRow = gmv + (size_t)(y0 + p0 - 1) * mbCols + x0;
+    uint32_t* nextUp = gmv + (size_t)(y0 + p0 + 31) * mbCols + x0;
     // Records of this lane's row; written by this warp's chain, so read
     // with coherent loads (never through the read-only path).
     MBRec* const rowRec = recs + (size_t)(y0 + min(ry, th - 1)) * mbCols + x0;
@@ -911,6 +891,7 @@ __global__ void __launch_bounds__(32 * kParseWarps) kParseMB(const FrameDesc* fr
   if (lane == 0) flags[k] = p.intra ? 1 : 0;
 }
 
+constexpr int kRowMax = 128;  // tiles at most this many macroblocks wide have their vectors in shared memory
 // The same wavefront for a tile of at most kRowMax macroblocks' width, by a
 // CTA: the records of a pass of 32 rows are read into shared memory by all
 // threads, one warp runs the wavefront there, and all threads write the
@@ -1010,10 +991,7 @@ __device__ void predictVectorsShared(const FrameDesc* fp, const TileRange& tr, i
 // wavefront.
 constexpr int kFlagsPerThread = 8;
 __global__ void __launch_bounds__(kFinishThreads) kTileFinish(const FrameDesc* frames, const int4* jobs, int njobs) {
-  __shared__ union {
-    WarpRows rows;
-    FinishVectors vectors;
-  } sV;
+  __shared__ FinishVectors sV;
   __shared__ int sWarp[kFinishThreads / 32];
   const int jb = blockIdx.x;
   if (jb >= njobs) return;
@@ -1056,8 +1034,8 @@ __global__ void __launch_bounds__(kFinishThreads) kTileFinish(const FrameDesc* f
   }
   if (tid == 0) fp->tileStat[tile].intraCount = base;
   if (!fp->inter) return;
-  if (tw <= kRowMax) predictVectorsShared(fp, tr, done, sV.vectors, tid);
-  else if (warp == 0) predictVectors(fp, tile, done, sV.rows, lane);
+  if (tw <= kRowMax) predictVectorsShared(fp, tr, done, sV, tid);
+  else if (warp == 0) predictVectors(fp, tile, done, lane);
 }
 
 // ---------------------------------------------------------------------------
