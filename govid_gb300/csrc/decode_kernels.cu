@@ -2233,7 +2233,9 @@ static void launchIntraW(const FrameDesc* frames, const int2* jobs, int njobs, i
 // maxTileKeys: the largest wavefront key range of its tiles (4*(w-1) +
 // 11*(h-1) + 1 for a tile of w x h macroblocks).  warps: the warps per CTA
 // (4, 8 or 16; anything else picks by the tile count: 16 up to one CTA per
-// SM, 8 up to two, else 4).
+// SM, 8 up to two, else 4).  Whatever their warps, a tile has two CTAs, one for
+// luma and one for chroma, while the tiles are at most half the SMs
+// (kIntraRecon says why), else one for both.
 void launchIntra(const FrameDesc* frames, const int2* jobs, int njobs, int maxTileMBs, int maxTileKeys, int warps,
                  cudaStream_t s) {
   if (njobs <= 0) return;
