@@ -36,9 +36,10 @@ Reported (one JSON line on rank 0):
 
 --impl reference times the reference's CPU decoder (the oracle restatement;
 Go is not available on the box) on all host cores for the same workload.  It
-loads neither the GPU library nor the encoder: its clip comes from the content
-cache (encoded by a child process when absent) and is demuxed by the oracle's
-own container parser.
+loads neither the GPU library nor the encoder, nor does a child process of it:
+its clip is kept encoded in the package (govid_gb300/clips; with another
+--frames it comes from the content cache, encoded by a child process when
+absent) and is demuxed by the oracle's own container parser.
 """
 from __future__ import annotations
 
@@ -903,7 +904,7 @@ def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return
-    from govid_gb300 import workloads  # content cache only: loads no native code
+    from govid_gb300 import workloads  # the clip only: loads no native code
 
     clip = workloads.load([workloads.single_1080(args.frames)], in_child=True)[0]
     sys.path.insert(0, str(ROOT / "oracle"))

@@ -17,10 +17,12 @@ Encoding is slow next to decoding (about 2 s of one host core per 1080p
 frame), so clips are cached on disk under ``EBIV_CONTENT_DIR`` (default: the
 ``.content_cache`` folder at the repository root) keyed by their parameters
 and by a hash of the encoder sources.  A missing clip is encoded by
-``python -m govid_gb300.workloads <names>`` in a child process, so that a
-process which must not load the decoder library (the CPU reference arm of the
-benchmark) can still obtain its input.  This module itself loads no native
-code unless it encodes.
+``python -m govid_gb300.workloads <names>`` in a child process.  This module
+itself loads no native code unless it encodes.
+
+``single_1080`` is kept encoded in the package (``clips/``): the benchmark's CPU
+reference arm decodes it, and a run of that arm in which any process maps this
+package's native library measures something else than the reference alone.
 """
 from __future__ import annotations
 
@@ -34,6 +36,7 @@ from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 ROOT = PKG.parent
+CLIPS = PKG / "clips"
 
 # Encoder settings are part of every cache key: a change to the encoder or the
 # scene generator invalidates the cached clips.
@@ -83,7 +86,8 @@ class Clip:
         return hashlib.sha1(k.encode()).hexdigest()[:20]
 
     def path(self) -> Path:
-        return content_dir() / f"{self.name}-{self.key()}.ebiv"
+        name = f"{self.name}-{self.key()}.ebiv"
+        return CLIPS / name if (CLIPS / name).exists() else content_dir() / name
 
     def describe(self) -> dict:
         return {"w": self.w, "h": self.h, "frames": self.frames, "seed": self.seed, "qp": self.qp, "gop": self.gop,
