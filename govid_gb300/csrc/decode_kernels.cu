@@ -596,54 +596,62 @@ __device__ __noinline__ int fullChain(const FrameDesc* fp, int tile, const Entro
   return k;
 }
 
-// The symbol chain of a tile from macroblock `from` on, by one thread (Chain).
-// Returns the macroblocks decoded, with *st behind the last one, and in *next
-// the first one behind those that it leaves to the full chain.  Where it
-// failed, the decoder's state is not known; a second run up to the last
-// macroblock that is surely complete finds it.
-__device__ __forceinline__ int symbolChain(const FrameDesc* fp, const TileRange& tr, const EntropyTables& sT,
-                                           ChainState* st, int from, int* next) {
-  const int tw = tr.mbX1 - tr.mbX0;
+// The symbol chain of a tile's macroblocks from `from` to `to`, into their logs.
+__device__ __forceinline__ bool runChain(Chain& d, const FrameDesc* fp, const TileRange& tr, const EntropyTables& sT,
+                                         const ChainState& st, int from, int to) {
   uint16_t* const log = reinterpret_cast<uint16_t*>(coefRegion(fp, tr.mbY0 * fp->mbCols + tr.mbX0));
-  int upTo = tw * (tr.mbY1 - tr.mbY0);
-  Chain d;
-#pragma unroll 1
-  while (!d.run(fp->pkt + tr.offset, *st, sT, fp->inter, from, upTo, log, kLogEntries, fp->symOff + tr.mbBase, tw,
-                fp->mbCols)) {
-    *next = d.mb + 1;
-    upTo = d.reached(from);
-    if (upTo == from) return from;
-  }
-  *st = d.state();
-  return upTo;
+  return d.run(fp->pkt + tr.offset, st, sT, fp->inter, from, to, log, kLogEntries, fp->symOff + tr.mbBase,
+               tr.mbX1 - tr.mbX0, fp->mbCols);
 }
 
-// A tile, by one warp: the symbol chain as far as it goes, the full chain for
-// the macroblocks that it leaves (one with no room for its log; one where a
-// symbol fails, which ends the tile), and so on.  A tile with an error takes
-// two passes of the symbol chain up to there, which are quicker together than
-// the full chain's one.
-__device__ __forceinline__ void decodeTile(const FrameDesc* fp, int tile, const EntropyTables& sT, int lane) {
+// A tile that the symbol chain left, by one warp: the symbol chain as far as
+// it goes, the full chain for the macroblocks that it leaves (one with no room
+// for its log; one where a symbol fails, which ends the tile), and so on.
+// Where the chain failed (f: in its run over the whole tile), the decoder's
+// state is not known; another run up to the last complete macroblock finds it.
+//
+// Two runs take 250 cycles a symbol where the full chain takes 340, and what
+// the first one lost in the macroblock where it failed another 125: they pay
+// when they got some way.  While it is not four times as far as what was lost,
+// as where macroblocks with no room for their log follow one another, the full
+// chain is left 1, 3, 7 and more macroblocks behind that one (hold).  Of 1, 2,
+// 4 and 8 times, 4 is the best or as good on frames at q0 to q6, by up to 3 %.
+// 920 macroblocks of 384 escapes each: 251 ms without this, 191 now.
+__device__ __noinline__ void leftTile(const FrameDesc* fp, int tile, const EntropyTables& sT, int lane, ChainFailure f) {
   const TileRange tr = fp->tiles[tile];
   const int tw = tr.mbX1 - tr.mbX0, total = tw * (tr.mbY1 - tr.mbY0);
-  uint32_t* const entries = fp->symOff + tr.mbBase;
-  for (int k = lane; k < total; k += 32) entries[k] = kSkipOffset;
-  __syncwarp();
   ChainState st = {0u, 0u, 0u, 0u, -1};
   if (tr.length >= (uint32_t)(kStates * 4)) st = initialState(fp->pkt + tr.offset, tr.length);
-  int done = 0;
+  int done = 0, hold = 0, upTo = f.reached;
   while (st.pos >= 0 && done < total) {
-    int next = 0;
-    if (lane == 0) done = symbolChain(fp, tr, sT, &st, done, &next);
+    if (lane == 0) {
+      const int start = st.pos;
+      Chain d;
+#pragma unroll 1
+      while (upTo > done) {
+        if (runChain(d, fp, tr, sT, st, done, upTo)) {
+          st = d.state();
+          break;
+        }
+        f = d.failure(done);
+        upTo = f.reached;
+      }
+      if (upTo < total) {
+        hold = start - st.pos >= 4 * (st.pos - f.pos) ? 0 : min(2 * hold + 1, 255);
+        f.next = min(total, f.next + hold);
+      }
+      done = upTo;
+    }
     done = __shfl_sync(kFull, done, 0);
     if (done == total) break;
-    next = __shfl_sync(kFull, next, 0);
+    f.next = __shfl_sync(kFull, f.next, 0);
     st.x0 = __shfl_sync(kFull, st.x0, 0);
     st.x1 = __shfl_sync(kFull, st.x1, 0);
     st.x2 = __shfl_sync(kFull, st.x2, 0);
     st.x3 = __shfl_sync(kFull, st.x3, 0);
     st.pos = __shfl_sync(kFull, st.pos, 0);
-    done = fullChain(fp, tile, sT, lane, &st, done, next);
+    done = fullChain(fp, tile, sT, lane, &st, done, f.next);
+    upTo = total;
   }
   const bool err = st.pos < 0;
   // Macroblocks the tile never reached are left untouched by reconstruction.
@@ -651,12 +659,29 @@ __device__ __forceinline__ void decodeTile(const FrameDesc* fp, int tile, const 
     MBRec* r = fp->mbrec + (size_t)(tr.mbY0 + k / tw) * fp->mbCols + tr.mbX0 + k % tw;
     r->mode = kRecNone;
     r->wmask = 0;
-    entries[k] = kDecodedOffset;
+    fp->symOff[tr.mbBase + k] = kDecodedOffset;
   }
   if (lane == 0) {
     fp->tileStat[tile] = TileStat{err ? kErrCorrupt : 0, 0, done, 0};
     if (err) atomicExch(fp->status, kErrCorrupt);
   }
+}
+
+// A tile, by one warp.
+__device__ __forceinline__ void decodeTile(const FrameDesc* fp, int tile, const EntropyTables& sT, int lane) {
+  const TileRange tr = fp->tiles[tile];
+  const int total = (tr.mbX1 - tr.mbX0) * (tr.mbY1 - tr.mbY0);
+  for (int k = lane; k < total; k += 32) fp->symOff[tr.mbBase + k] = kSkipOffset;
+  __syncwarp();
+  ChainFailure f = {0, 0, 0};
+  bool whole = false;
+  if (lane == 0 && tr.length >= (uint32_t)(kStates * 4)) {
+    Chain d;
+    whole = runChain(d, fp, tr, sT, initialState(fp->pkt + tr.offset, tr.length), 0, total);
+    if (whole) fp->tileStat[tile] = TileStat{0, 0, total, 0};
+    else f = d.failure(0);
+  }
+  if (!__shfl_sync(kFull, whole ? 1 : 0, 0)) leftTile(fp, tile, sT, lane, f);
 }
 
 // Entropy jobs: up to kEntropyWarps tiles of one frame per job, one warp per

@@ -172,6 +172,11 @@ struct ChainState {
   uint32_t x0, x1, x2, x3;
   int32_t pos;
 };
+// Where a run of the symbol chain failed: the macroblocks surely complete, the
+// first one behind those that it leaves, and the stream bytes left.
+struct ChainFailure {
+  int reached, next, pos;
+};
 // The state at a tile's start, from the end of its len >= 16 bytes
 // (ransDecoder.reset, ebiv/rans.go:236-250).
 EBIV_DEV ChainState initialState(const uint8_t* buf, uint32_t len) {
@@ -684,7 +689,7 @@ struct Chain {
   // frame `stride` macroblocks wide, of which tileLog holds the tile's first.
   // offsets (kSkipOffset everywhere before) gets the first entry of each
   // macroblock that is not skip, with a tile width the number of its entries.
-  // False when macroblocks from reached() on are left to the full chain: a
+  // False when macroblocks (failure()) are left to the full chain: a
   // symbol failed, or there was no room for the most entries that could follow.
   EBIV_DEV bool run(const uint8_t* buf, const ChainState& s, const EntropyTables& tables, int inter, int from, int total,
                     uint16_t* tileLog, int entries, uint32_t* offsets, int tileWidth = 0, int stride = 0) {
@@ -738,11 +743,12 @@ struct Chain {
   }
   // After run(): where the decoder stands behind the last macroblock.
   EBIV_DEV ChainState state() const { return ChainState{x0, x1, x2, x3, rem >> 3}; }
-  // After a run() from macroblock `from` on that failed in macroblock mb: the
-  // macroblocks surely complete.  In a frame of intra macroblocks only, the
-  // failing symbol may be up to three before the one where that was noticed,
-  // at the end of the macroblock before.
-  EBIV_DEV int reached(int from) const { return intraOnly && mb > from ? mb - 1 : mb; }
+  // After a run() from macroblock `from` on that failed.  In a frame of intra
+  // macroblocks only, the failing symbol may be up to three before the one
+  // where that was noticed, at the end of the macroblock before.
+  EBIV_DEV ChainFailure failure(int from) const {
+    return ChainFailure{intraOnly && mb > from ? mb - 1 : mb, mb + 1, rem >> 3};
+  }
 };
 
 }  // namespace dev

@@ -79,8 +79,8 @@ const char* sameRooms(const PayloadPlan& p, const TileRange& r, const uint8_t* p
     bool again = false;
     while (!d.run(buf, st, tables, inter, done, upTo, rooms.at(r.mbX0, r.mbY0), kRoom, entries.data(), tw, geo.mbCols)) {
       if (again) return "the second run failed";
-      next = d.mb + 1;
-      upTo = d.reached(done);
+      next = d.failure(done).next;
+      upTo = d.failure(done).reached;
       if (upTo < done || upTo >= next || next - upTo > 2) return "no progress";
       if (upTo == done) break;
       again = true;

@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 W, H = 640, 368
 
 
-def _key(seed=3, most=60, full=()):
+def _key(seed=3, most=60, full=(), least=3):
     """A key frame of one tile, about 100 symbols a macroblock: its chain is nearly all of its decode's time.  The
     macroblocks of `full` have all of their coefficients and many escapes, more than their log has room for."""
     rng = np.random.default_rng(seed)
@@ -25,7 +25,7 @@ def _key(seed=3, most=60, full=()):
     at = rng.integers(0, 384, (mbs, most))
     levels[np.arange(mbs)[:, None], at] = rng.integers(-3, 4, (mbs, most))
     for m in full:
-        levels[m] = rng.choice([-1, 1], 384) * rng.integers(3, 9, 384)
+        levels[m] = rng.choice([-1, 1], 384) * rng.integers(least, 9, 384)
     return ebiv.encode_key_from_levels(W, H, 20, 0, levels)
 
 
@@ -97,6 +97,16 @@ def test_what_the_chain_leaves_costs_one_pass_more(gpu_required, what):
     assert _status(codec, pkt) == st == (ebiv.ErrCorrupt.status if what == "error" else 0)
     if st == 0:
         assert codec.decode(pkt).packed() == planes
+
+
+def test_full_macroblocks_in_a_row_are_not_tried_one_by_one(gpu_required):
+    # 920 macroblocks of 384 escapes each: the full chain by itself takes 11.2 times the time of the symbol chain for
+    # the plain frame; 14.2 times when every macroblock is tried by the symbol chain first.  In between lies 12.7.
+    codec = ebiv.Codec()
+    plain, full = _key(), _key(full=range((W // 16) * (H // 16)), least=5)
+    a, b = _ms(lambda: codec.decode(plain)), _ms(lambda: codec.decode(full), 3)
+    assert b < 12.7 * a, f"plain {a:.2f} ms, full {b:.2f} ms"
+    assert codec.decode(full).packed() == ebiv_oracle.decode_all([full])[0][1]
 
 
 @pytest.mark.parametrize("lookahead,depth", [(1, 0), (4, 0), (4, 2)])
