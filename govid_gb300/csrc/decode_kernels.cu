@@ -125,7 +125,16 @@ struct WarpChain {
       e = entryAt(q);
       for (uint4 n = entryAt(q += 16); (x & (kM - 1)) >= n.y; n = entryAt(q += 16)) e = n;
     }
-    uint32_t xn = e.x * (x >> kScaleBits) + x - e.y;
+    return renew(e.x * (x >> kScaleBits) + x - e.y, (int)((e.w >> kLogShift) & 15u));
+  }
+  // A symbol of ctxBypass, whose two symbols have half of the range each
+  // (installBypass, ebiv/rans.go:317-322).
+  __device__ __forceinline__ int bypass() {
+    if (err) return 0;
+    return renew((x0 >> kScaleBits << (kScaleBits - 1)) + (x0 & (kM / 2 - 1)), (int)(x0 >> (kScaleBits - 1) & 1u));
+  }
+  // Stream bytes for the state behind symbol s, which it returns.
+  __device__ __forceinline__ int renew(uint32_t xn, int s) {
     if (xn < kLower) {
       if (pos >= 2 && xn >= (kLower >> 16)) {
         if (xn < (kLower >> 8)) {  // two bytes
@@ -153,7 +162,7 @@ struct WarpChain {
     x1 = x2;
     x2 = x3;
     x3 = xn;
-    return (int)((e.w >> kLogShift) & 15u);
+    return s;
   }
   __device__ __forceinline__ int sym(int ctx) { return symAt(rowOf(ctx)); }
   // Takes up a tile's decoding (b: its bytes).
@@ -176,7 +185,7 @@ struct WarpChain {
 __device__ __forceinline__ uint32_t classValue(WarpChain& d, int classCtx) {
   const int cls = d.sym(classCtx);
   uint32_t v = (uint32_t)min(cls, 1);
-  for (int i = 1; i < cls; i++) v = v << 1 | (uint32_t)d.sym(ctxBypass);
+  for (int i = 1; i < cls; i++) v = v << 1 | (uint32_t)d.bypass();
   return v;
 }
 __device__ __forceinline__ int unzigzag(uint32_t u) { return (int)(u >> 1) ^ -(int)(u & 1); }
@@ -616,7 +625,7 @@ __device__ __forceinline__ bool runChain(Chain& d, const FrameDesc* fp, const Ti
 // as where macroblocks with no room for their log follow one another, the full
 // chain is left 1, 3, 7 and more macroblocks behind that one (hold).  Of 1, 2,
 // 4 and 8 times, 4 is the best or as good on frames at q0 to q6, by up to 3 %.
-// 920 macroblocks of 384 escapes each: 251 ms without this, 191 now.
+// 920 macroblocks of 384 escapes each: 251 ms without this, 167 now.
 __device__ __noinline__ void leftTile(const FrameDesc* fp, int tile, const EntropyTables& sT, int lane, ChainFailure f) {
   const TileRange tr = fp->tiles[tile];
   const int tw = tr.mbX1 - tr.mbX0, total = tw * (tr.mbY1 - tr.mbY0);
