@@ -571,8 +571,7 @@ __device__ __forceinline__ int decodeMB(WarpChain& d, int inter, MBRec* rec, uin
 
 // A macroblock's log, and the same as 16-byte words: its coefficient region.
 constexpr int kLogEntries = kSymPerMB / 2, kLogWords = kSymPerMB / 16;
-static_assert(kSymPerMB % 16 == 0 && kHeaderEntries + blockEntries(16, 256) + kLastEntries <= kLogEntries,
-              "a macroblock's log");
+static_assert(kSymPerMB % 16 == 0 && kPlainMBEntries + kLastEntries <= kLogEntries, "a macroblock's log");
 __device__ __forceinline__ uint32_t* coefRegion(const FrameDesc* fp, int idx) {
   return fp->coef + (size_t)idx * kCoefPerMB;
 }
@@ -606,7 +605,7 @@ __device__ __noinline__ int fullChain(const FrameDesc* fp, int tile, const Entro
 }
 
 // The symbol chain of a tile's macroblocks from `from` to `to`, into their logs.
-__device__ __forceinline__ bool runChain(Chain& d, const FrameDesc* fp, const TileRange& tr, const EntropyTables& sT,
+__device__ __forceinline__ bool runChain(ChainOf<true>& d, const FrameDesc* fp, const TileRange& tr, const EntropyTables& sT,
                                          const ChainState& st, int from, int to) {
   uint16_t* const log = reinterpret_cast<uint16_t*>(coefRegion(fp, tr.mbY0 * fp->mbCols + tr.mbX0));
   return d.run(fp->pkt + tr.offset, st, sT, fp->inter, from, to, log, kLogEntries, fp->symOff + tr.mbBase,
@@ -635,7 +634,7 @@ __device__ __noinline__ void leftTile(const FrameDesc* fp, int tile, const Entro
   while (st.pos >= 0 && done < total) {
     if (lane == 0) {
       const int start = st.pos;
-      Chain d;
+      ChainOf<true> d;
 #pragma unroll 1
       while (upTo > done) {
         if (runChain(d, fp, tr, sT, st, done, upTo)) {
@@ -685,7 +684,7 @@ __device__ __forceinline__ void decodeTile(const FrameDesc* fp, int tile, const 
   ChainFailure f = {0, 0, 0};
   bool whole = false;
   if (lane == 0 && tr.length >= (uint32_t)(kStates * 4)) {
-    Chain d;
+    ChainOf<true> d;
     whole = runChain(d, fp, tr, sT, initialState(fp->pkt + tr.offset, tr.length), 0, total);
     if (whole) fp->tileStat[tile] = TileStat{0, 0, total, 0};
     else f = d.failure(0);

@@ -53,7 +53,7 @@ constexpr int kEntropyTilesPerJob = 4;
 // it writes the levels there, so the log takes no memory of its own.  816
 // entries of two bytes: key frames coded at q18 average about 125 a macroblock,
 // small textured ones at q22 185; 384 nonzero coefficients without an escape
-// take 843.
+// take at most 806.
 constexpr int kSymPerMB = 4 * kCoefPerMB;
 
 struct TileStat {

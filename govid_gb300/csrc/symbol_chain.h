@@ -106,15 +106,17 @@ constexpr int kLogShift = 8;
 constexpr uint32_t kLogNonzero = 4;               // token flag, where Chain::far looks
 constexpr uint32_t kSkipOffset = 0xFFFFFFFFu;     // a skip macroblock: it has no log
 constexpr uint32_t kDecodedOffset = 0xFFFFFFFEu;  // one that the full chain has decoded, or that is not reached
-// The entries of a macroblock's header (mode, reference, partition, eight
-// vector components, pattern, transform size), the most that n blocks with
-// `coefs` coefficients take without escapes (a token and a sign for each
-// coefficient, the mode, end and last sign of each block) and what an escape
-// adds (its value).  The most of a macroblock are all of these together.
+// The most entries of a block of n positions (the mode in front is one): a
+// token and a sign for each position and the end; a block has a last sign only
+// when its nonzero tokens are four at most, so that others have no sign.  Of a
+// macroblock without escapes: the header (mode, reference, partition, eight
+// vector components, pattern, transform size) and the blocks, 17 with a mode.
+// An escape adds its value.
+EBIV_DEV constexpr int blockEntries(int n) { return 2 * n + 1; }
 constexpr int kHeaderEntries = 5 + 8 * 2, kEscapeEntries = 2;
-EBIV_DEV constexpr int blockEntries(int n, int coefs) { return 3 * n + 2 * coefs; }
+constexpr int kPlainMBEntries = kHeaderEntries + 2 * 384 + 17;
 constexpr int kLastEntries = 4;  // kept free: the next macroblock's transform size, once
-constexpr int kMBEntries = kHeaderEntries + 3 * 18 + (2 + kEscapeEntries) * 384 + kLastEntries;
+constexpr int kMBEntries = kPlainMBEntries + kEscapeEntries * 384 + kLastEntries;
 
 // The entry of symbol s of context c, which starts at st and has frequency
 // freq, in a row that keeps class cls (signs).
@@ -213,7 +215,11 @@ EBIV_DEV ChainState initialState(const uint8_t* buf, uint32_t len) {
 // next entry's load before the test instead of after it: 107 on the line; four
 // symbols to a test: 70, but what follows an end in its group is lost and
 // undone, 170 with everything.
-struct Chain {
+//
+// kRooms: the macroblocks' logs lie in rooms of their own, as the kernel has
+// them in the coefficient regions, else one behind the other.
+template <bool kRooms>
+struct ChainOf {
   uint32_t x0, x1, x2, x3;  // states in use order: x0 decodes the next symbol
   // The stream, read backwards: hi and lo are its next words, off the bits of
   // hi that are used, nw the word after lo, wp its address; rem counts the
@@ -224,16 +230,15 @@ struct Chain {
   const uint32_t* wp;
   int32_t rem;
   const EntropyTables* t;
-  // The log.  With width 0 the entries of all macroblocks follow one another;
-  // else each macroblock has `pitch` of its own, the tile's rows (of `width`)
-  // lie `gap` more than theirs apart, and log moves on by that with the rows:
-  // macroblock mb, before rowEnd, has those from log + mb * pitch.  room: what
-  // the macroblock has left when its open kind of blocks takes the most.
+  // The log of `entries` entries, or rooms of as many: the tile's rows (of
+  // `width`) lie `gap` more than their rooms apart, and log moves on by that
+  // with the rows; macroblock mb, before rowEnd, has those from log + mb *
+  // entries.
   uint16_t* log;
   uint16_t* lp;     // the next entry
   uint16_t* first;  // the macroblock's first one
-  uint16_t* end;    // the end of what it, or the tile, has
-  int32_t width, pitch, gap, rowEnd, room;
+  int32_t width, entries, gap, rowEnd;
+  int32_t escaped;  // the macroblock has an escape
   int32_t stop;    // macroblocks to decode; 0 after a failure
   // The grammar inside a macroblock's blocks.  kind: its block entry; left:
   // the blocks after this one that have the same, -1 past the macroblock's
@@ -246,9 +251,8 @@ struct Chain {
   // position after the first nonzero token's and before this one (unary, the
   // oldest lost).  far: bit 2 is set once a nonzero token was kSDHMinSpan or
   // more positions after the first.
-  // The macroblocks: mb is the current one, mbOff where their logs begin
-  // (width 0) or how many entries they have; intraOnly: no mode in front of a
-  // macroblock.
+  // The macroblocks: mb is the current one, mbOff where their logs begin or
+  // how many entries they have; intraOnly: no mode in front of a macroblock.
   uint4 kind;
   int32_t left;
   int32_t mb;
@@ -276,20 +280,36 @@ struct Chain {
   // A symbol that cannot be decoded (an unused context, a byte before the
   // tile's first), or one with no room: the tile is left to the full chain.
   EBIV_DEV void fail() { stop = 0; }
-  // The log's part for macroblock mb, from lp on with width 0.
+  // The log's part for macroblock mb.
   EBIV_DEV void open() {
-    if (width) {
+    if (kRooms) {
       while (mb >= rowEnd) {
         rowEnd += width;
         log += gap;
       }
-      lp = log + (ptrdiff_t)mb * pitch;
-      end = lp + pitch;
+      lp = log + (ptrdiff_t)mb * entries;
     }
     first = lp;
+    escaped = 0;
   }
   // All of macroblock mb is in the log.
-  EBIV_DEV void close() { mbOff[mb] = (uint32_t)(width ? lp - first : first - log); }
+  EBIV_DEV void close() { mbOff[mb] = (uint32_t)(kRooms ? lp - first : first - log); }
+  // And the next one follows (without a branch).
+  EBIV_DEV void step() {
+    close();
+    mb++;
+    if (kRooms) {
+      const bool row = mb == rowEnd;
+      rowEnd += row ? width : 0;
+      log += row ? gap : 0;
+      first += row ? entries + gap : entries;
+      lp = first;
+    }
+    first = lp;
+    escaped = 0;
+  }
+  // The entries left from lp on.
+  EBIV_DEV int room() const { return entries - (int)(lp - (kRooms ? first : log)); }
   // Keeps off below 32.
   EBIV_DEV void refill() {
 #ifdef __CUDACC__  // without a branch
@@ -403,18 +423,20 @@ struct Chain {
     bands = __funnelshift_r(bands, 0u, adv);
   }
 
-  // The blocks of the queue's next byte, when the log has room for them behind
-  // the entry lp[j].
+  // The blocks of the queue's next byte, behind the entry lp[j].  Without an
+  // escape before it in the macroblock there is room for them.
   EBIV_DEV void nextKind(int j) {
     kind = entryAt((uint32_t)offsetof(EntropyTables, block) - 16 + 16 * (queue & 15u));
     left = (int32_t)((queue >> 4) & 15u);
-    const int most = (queue & 3u) != 0 ? blockEntries(left + 1, 256) : blockEntries(left + 1, 64 * (left + 1));
     queue >>= 8;
-    room = (int32_t)(end - lp) - (j + 1) - most - kLastEntries;
-    if (room < 0) {
+    if (escaped && room() - (j + 1) < (left + 1) * blockEntries(positions(kind.y)) + kLastEntries) {
       fail();
       left = -1;
     }
+  }
+  // Up to the edge and behind it: the positions of a block whose z or kind is at v.
+  EBIV_DEV int positions(uint32_t v) const {
+    return 2048 - (int)(v >> 20) + (v & kERest ? 2048 - (int)(kind.w >> 20) : 0);
   }
   // The blocks of an intra macroblock of transform size tx.
   static EBIV_DEV uint32_t intraQueue(uint32_t tx) {
@@ -427,13 +449,11 @@ struct Chain {
     if ((e.w & kLogKind) == kLogValue) {
       queue = intraQueue(min((e.w >> kLogShift) & 15u, 2u));  // alphabet size 3
       lp += j;
-      close();
-      mb++;
-      open();
+      step();
       *lp = (uint16_t)e.w;
       lp -= j;
     } else if (queue == 0) {
-      if (!intraOnly || mb + 1 >= stop) return;
+      if (!intraOnly || mb + 1 >= stop || (!kRooms && room() < kPlainMBEntries + 2 * kLastEntries)) return;
       kind = make_uint4(rowOf(ctxTxSize), 0u, 0u, 0u);
       left = 0;
       return;
@@ -460,7 +480,6 @@ struct Chain {
   EBIV_DEV void tokens(uint32_t blocks) {
     queue = blocks;
     nextKind(-1);
-    if (left < 0) return;
     z = kind.y;
     bands = kind.z;
     seen = kClassMask;
@@ -591,8 +610,9 @@ struct Chain {
         // A failure, or an escape: its value, then the sign unless it is the
         // first nonzero token.
         e = symbolOf(e);
-        room -= kEscapeEntries;
-        if (room < 0) return fail();
+        escaped = 1;
+        if (room() < kEscapeEntries + blockEntries(positions(z)) + left * blockEntries(positions(kind.y)) + kLastEntries)
+          return fail();
         put(e.w);
         putValue(classValue(ctxEscClass));
         if (seen & kGroupMask) put(kLogSign | sym(ctxSign) << kLogShift);
@@ -679,23 +699,22 @@ struct Chain {
 
   // The chain of a whole tile: len bytes at buf, its log into tileLog.
   EBIV_DEV bool run(const uint8_t* buf, uint32_t len, const EntropyTables& tables, int inter, int total,
-                    uint16_t* tileLog, int entries, uint32_t* offsets, int tileWidth = 0, int stride = 0) {
+                    uint16_t* tileLog, int logEntries, uint32_t* offsets, int tileWidth = 0, int stride = 0) {
     return len >= (uint32_t)(kStates * 4) &&
-           run(buf, initialState(buf, len), tables, inter, 0, total, tileLog, entries, offsets, tileWidth, stride);
+           run(buf, initialState(buf, len), tables, inter, 0, total, tileLog, logEntries, offsets, tileWidth, stride);
   }
   // The chain of a tile's macroblocks from `from` on, where its decoder stands
   // at s, up to macroblock `total`.  Its log goes into tileLog, which has
-  // `entries` entries, or with a tile width as many for each macroblock of a
-  // frame `stride` macroblocks wide, of which tileLog holds the tile's first.
-  // offsets (kSkipOffset everywhere before) gets the first entry of each
-  // macroblock that is not skip, with a tile width the number of its entries.
+  // logEntries entries, or as many for each macroblock (kRooms; the tile is
+  // tileWidth macroblocks wide, the frame `stride`, and tileLog the room of the
+  // tile's first).  offsets (kSkipOffset everywhere before) gets the first entry
+  // of each macroblock that is not skip, or the number of its entries (kRooms).
   // False when macroblocks (failure()) are left to the full chain: a
   // symbol failed, or there was no room for the most entries that could follow.
   EBIV_DEV bool run(const uint8_t* buf, const ChainState& s, const EntropyTables& tables, int inter, int from, int total,
-                    uint16_t* tileLog, int entries, uint32_t* offsets, int tileWidth = 0, int stride = 0) {
-    log = lp = tileLog;
-    end = log + entries;
-    pitch = entries;
+                    uint16_t* tileLog, int logEntries, uint32_t* offsets, int tileWidth = 0, int stride = 0) {
+    log = lp = first = tileLog;
+    entries = logEntries;
     width = rowEnd = tileWidth;
     gap = (stride - tileWidth) * entries;
     mbOff = offsets;
@@ -711,7 +730,7 @@ struct Chain {
         if (mode == mbSkip) break;
       }
       open();
-      if (end - lp < kHeaderEntries + kLastEntries) return false;
+      if (!kRooms && room() < kPlainMBEntries + kLastEntries) return false;
       if (inter) put(kLogValue | mode << kLogShift);
       uint32_t cbp = kNumCBP - 1;
       if (mode != mbIntra) {
@@ -750,6 +769,7 @@ struct Chain {
     return ChainFailure{intraOnly && mb > from ? mb - 1 : mb, mb + 1, rem >> 3};
   }
 };
+using Chain = ChainOf<false>;
 
 }  // namespace dev
 }  // namespace ebiv

@@ -75,7 +75,7 @@ const char* sameRooms(const PayloadPlan& p, const TileRange& r, const uint8_t* p
   long left = 0;
   while (done < total) {
     int upTo = total, next = 0;
-    dev::Chain d;
+    dev::ChainOf<true> d;
     bool again = false;
     while (!d.run(buf, st, tables, inter, done, upTo, rooms.at(r.mbX0, r.mbY0), kRoom, entries.data(), tw, geo.mbCols)) {
       if (again) return "the second run failed";
