@@ -12,10 +12,11 @@
         frames, lookahead 1): the batched stages;
     python -m govid_gb300.profile_cases helpers
         the alt-ref filter over 16 1080p frames, then forwardDCT + satd of
-        262144 8x8 blocks.
+        262144 8x8 blocks, then the motion net's candidates and the exhaustive
+        search for a 1920x1088 pair.
 
-Every case checks its statuses; the decode cases use the content cache
-(govid_gb300/workloads.py).
+Every case checks its statuses; the decode cases use the clips of
+govid_gb300/workloads.py.
 """
 from __future__ import annotations
 
@@ -24,7 +25,7 @@ import sys
 
 import numpy as np
 
-from . import ebiv, workloads
+from . import ebiv, mvnet, workloads
 
 
 def _clip(frames: int) -> list[bytes]:
@@ -76,6 +77,10 @@ def helpers() -> None:
     a.build(frames, 1920, 1080, 16)
     blocks = np.random.default_rng(1).integers(-255, 256, size=(1 << 18, 8, 8), dtype=np.int64).astype(np.int32)
     ebiv.BlockAnalysis().fdct_satd(blocks)
+    cur, ref = (np.pad(mvnet.luma(f, 1920, 1080), ((0, 8), (0, 0)), mode="edge") for f in frames[:2])
+    net = mvnet.MvNet(1920, 1088).load()
+    net.propose(cur, ref)
+    net.exhaustive(cur, ref)
     print("altref accepted", a.accepted)
 
 
