@@ -2,11 +2,12 @@
 //
 // Stage A  kEntropy   one warp per tile, up to four tiles of one frame per
 //                     CTA sharing the frame's symbol tables: one thread runs
-//                     the tile's symbol chain (symbol_chain.h) into a log,
-//                     from which kParseMB makes one MBRec per macroblock plus
-//                     sparse levels; a tile that the chain leaves (a symbol
-//                     fails, the log is full) is decoded by the whole warp in
-//                     lockstep, records and levels included (fullChain).
+//                     the tile's symbol chain (symbol_chain.h) into the
+//                     macroblocks' logs, from which kParseMB makes one MBRec
+//                     per macroblock plus sparse levels; macroblocks that the
+//                     chain leaves (a symbol fails, no room for the log) are
+//                     decoded by the whole warp in lockstep, records and
+//                     levels included (leftTile, fullChain).
 // Stage B1 kInterRecon one warp per macroblock of an inter frame: motion
 //                     compensation (ebiv/motioncomp.go) from the last or
 //                     golden reference plus dequantized inverse DCT residual
@@ -721,10 +722,10 @@ __global__ void __launch_bounds__(32 * kEntropyWarps, 2) kEntropy(const FrameDes
   }
 }
 
-// Rebuilds the records of the logged macroblocks, one warp
-// per macroblock over every macroblock of the launch's tiles (grid.x: job *
-// kEntropyTilesPerJob + tile within the job; grid.y * kParseWarps: the
-// macroblock's raster index within its tile).  A skip macroblock's record is
+// Rebuilds the records of the logged macroblocks, one warp per macroblock over
+// every macroblock of the launch's tiles (grid.x: job * kEntropyTilesPerJob +
+// tile within the job; grid.y * kParseWarps: the macroblock's raster index
+// within its tile).  A skip macroblock's record is
 // fixed; of another one the warp takes the log out of the macroblock's
 // coefficient region into shared memory, whole, before it writes levels there;
 // then all of it reads the header, and each lane one log entry at a time of

@@ -65,8 +65,8 @@ namespace dev {
 constexpr uint32_t kEStop = 1u << 31, kEEnd = 1u << 30, kEImpure = 1u << 29, kEUnused = 1u << 28, kEBlock = 1u << 27;
 constexpr uint32_t kGroupBytes = 4096, kClassBytes = 16, kBucketMask = 0xFC0, kClassMask = 0x30;
 constexpr uint32_t kGroupMask = 0x1F000;                         // the group in a row
-constexpr uint32_t kERest = 1u << 8;                             // Chain::z: the edge is not the block's end
-constexpr uint32_t kECount = 1u << 20;                           // one position, in Chain::z
+constexpr uint32_t kERest = 1u << 8;                             // ChainOf::z: the edge is not the block's end
+constexpr uint32_t kECount = 1u << 20;                           // one position, in ChainOf::z
 constexpr uint32_t kEAdvance = kECount | kGroupBytes | 1u;       // a position, a band's step, a shift by one
 constexpr uint32_t kENonzero = 1u << 31 | kGroupMask | kEAdvance;
 constexpr int kTokenGroups = 4 * kNumBands;
@@ -75,7 +75,7 @@ constexpr int kSymbols = 18;  // own entries of a context: its symbols, then sen
 static_assert(kNumContexts == ctxTokenBase + 3 * kTokenGroups && ctxTokenBase <= kTokenGroups && kTokenGroups < 32,
               "entry layout");
 // What follows a block: the row of the next one's first symbol (x), the values
-// that Chain::z and Chain::bands start with (y, z) and z's count past position
+// that ChainOf::z and ::bands start with (y, z) and z's count past position
 // 19 (w), for blocks of a kind.  Kinds 0-2: luma by transform size, 3 chroma,
 // + 4 with an intra mode in front.
 constexpr int kBlockKinds = 8;
@@ -84,7 +84,7 @@ struct EntropyTables {
   uint4 symbol[kNumContexts * kSymbols];
   uint4 block[kBlockKinds];
 };
-static_assert(kSDHMinSpan == 4, "bit 2 of Chain::since");
+static_assert(kSDHMinSpan == 4, "bit 2 of ChainOf::since");
 // The row of context c (of the signs: with class 0 to keep).
 EBIV_DEV uint32_t rowOf(int c) {
   if (c == ctxSign) return kSignRow;
@@ -103,7 +103,7 @@ EBIV_DEV uint32_t rowOf(int c) {
 // values of 15 bits) are two entries of eight bits, the high ones first.
 constexpr uint32_t kLogToken = 0, kLogSign = 1u << 6, kLogMode = 2u << 6, kLogValue = 3u << 6, kLogKind = 3u << 6;
 constexpr int kLogShift = 8;
-constexpr uint32_t kLogNonzero = 4;               // token flag, where Chain::far looks
+constexpr uint32_t kLogNonzero = 4;               // token flag, where ChainOf::far looks
 constexpr uint32_t kSkipOffset = 0xFFFFFFFFu;     // a skip macroblock: it has no log
 constexpr uint32_t kDecodedOffset = 0xFFFFFFFEu;  // one that the full chain has decoded, or that is not reached
 // The most entries of a block of n positions (the mode in front is one): a
@@ -211,7 +211,7 @@ EBIV_DEV ChainState initialState(const uint8_t* buf, uint32_t len) {
 // join it again (one for each state, so that no register moves); escapes,
 // edges and second stream bytes leave it.  Measured: 91 cycles a symbol on the
 // line, 105 to 120 with everything (720p key frame of one tile at q18, 448
-// thousand symbols: 61 ms before, 26 ms), 31 a skip (77 before).  Issuing the
+// thousand symbols: 61 ms before, 25 ms), 31 a skip (77 before).  Issuing the
 // next entry's load before the test instead of after it: 107 on the line; four
 // symbols to a test: 70, but what follows an end in its group is lost and
 // undone, 170 with everything.
@@ -278,7 +278,7 @@ struct ChainOf {
     put(kLogValue | (v & 255u) << kLogShift);
   }
   // A symbol that cannot be decoded (an unused context, a byte before the
-  // tile's first), or one with no room: the tile is left to the full chain.
+  // tile's first), or one with no room: the macroblock is left to the full chain.
   EBIV_DEV void fail() { stop = 0; }
   // The log's part for macroblock mb.
   EBIV_DEV void open() {

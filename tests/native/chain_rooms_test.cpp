@@ -19,8 +19,9 @@ using dev::ChainState;
 
 constexpr int kRoom = kSymPerMB / 2;
 constexpr uint16_t kUntouched = 0xBEEF;
-// A macroblock of at most this many entries always has room: 21 of its header,
-// then at most 560 without escapes, and 115 escapes more (345 entries) fit.
+// A macroblock of at most this many entries always has room, however many of
+// them are escapes: behind u entries of a 16x16 block's escapes, four each,
+// there are u / 4 positions done, and the rest takes 515 - u / 2 at most.
 constexpr int kAlwaysFits = 345;
 
 struct Rooms {
