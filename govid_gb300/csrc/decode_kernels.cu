@@ -625,7 +625,8 @@ __device__ __forceinline__ bool runChain(ChainOf<true>& d, const FrameDesc* fp, 
 // as where macroblocks with no room for their log follow one another, the full
 // chain is left 1, 3, 7 and more macroblocks behind that one (hold).  Of 1, 2,
 // 4 and 8 times, 4 is the best or as good on frames at q0 to q6, by up to 3 %.
-// 920 macroblocks of 384 escapes each: 251 ms without this, 167 now.
+// 920 macroblocks of 384 escapes each: 251 ms without this, 169 now (and bypass
+// symbols without a table).
 __device__ __noinline__ void leftTile(const FrameDesc* fp, int tile, const EntropyTables& sT, int lane, ChainFailure f) {
   const TileRange tr = fp->tiles[tile];
   const int tw = tr.mbX1 - tr.mbX0, total = tw * (tr.mbY1 - tr.mbY0);
