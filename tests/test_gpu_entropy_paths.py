@@ -125,3 +125,48 @@ def test_more_jobs_than_ctas_of_several_frames(gpu_required, lookahead, depth):
     for r in b.drain():
         got[r.frame_index] = (r.status, b.download(r, 640, 400))
     assert [got[i] for i in range(len(pkts))] == want
+
+
+def _damaged(stream, rng):
+    """Tile bytes of some packets flipped, cleared or replaced (the tables in front of them mostly stay)."""
+    out = []
+    for p in stream:
+        b = bytearray(p)
+        at = int(rng.integers(min(len(b) - 1, 150), len(b)))
+        kind = int(rng.integers(0, 4))
+        if kind == 0:
+            b[at] ^= 1 << int(rng.integers(0, 8))
+        elif kind == 1:
+            b[at:] = bytes(len(b) - at)
+        elif kind == 2:
+            n = len(b[at:at + 30])
+            b[at:at + n] = rng.integers(0, 256, n, dtype=np.uint8).tobytes()
+        out.append(bytes(b))
+    return out
+
+
+@pytest.mark.parametrize("q,tiles", [(0, (1, 1)), (2, (2, 2)), (6, (2, 1))])
+def test_left_macroblocks_and_errors_match_the_oracle(gpu_required, q, tiles):
+    # High quality: macroblocks with and without room for their log beside one another, in key and inter frames;
+    # then with damaged tiles, whose errors come before, in and behind such macroblocks.
+    rng = np.random.default_rng(40 + q)
+    spec = ebiv.SceneSpec(width=160, height=96, seed=5 + q, sprites=6, noise_y16=90, noise_c16=60)
+    cont = ebiv.encode_scene(spec, 5, qp=q, gop=4, tiles=tiles, fast=True, threads=4)
+    clip = [p.data for p in ebiv.Reader(cont).packets()]
+    failing = 0
+    for k in range(16):
+        pkts = clip if k == 0 else _damaged(clip, rng)
+        want = [(st, planes if st == 0 else None) for st, planes in ebiv_oracle.decode_all(pkts)]
+        failing += sum(st != 0 for st, _ in want)
+        codec = ebiv.Codec()
+        assert [_status(codec, p) for p in pkts] == [st for st, _ in want], k
+        b = ebiv.Batch(lookahead=3, pipeline=k % 2)
+        b.add_stream(pkts)
+        res = {}
+        for _ in range(3 * len(pkts) + 6):
+            for r in b.round():
+                res[r.frame_index] = (r.status, b.download(r, 160, 96) if r.status == 0 else None)
+        for r in b.drain():
+            res[r.frame_index] = (r.status, b.download(r, 160, 96) if r.status == 0 else None)
+        assert [res[i] for i in range(len(pkts))] == want, k
+    assert failing > 10
